@@ -43,6 +43,59 @@ __host__ __device__ inline float clampf(float x, float lo, float hi) {
     return x;
 }
 
+// Correctly rounded f32 square root and quotients without the branches of the
+// general operators (whose special-case paths keep neighboring roots and
+// divisions from overlapping), for operands well inside the normal range.
+
+// Smallest and largest magnitude the functions below take: every product and
+// residual in them is then normal, so the residuals are exact.
+constexpr float PLAIN_MIN = 8.27180613e-25f;  // 2^-80
+constexpr float PLAIN_MAX = 1.20892582e+24f;  // 2^80
+
+#ifdef __CUDACC__
+// 1 / sqrt(a) and 1 / b to about an ulp (PTX approximations), a, b normal.
+__device__ inline float rsqrt_rough(float a) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+    return y;
+}
+
+// RN(sqrt(a)) for a in [PLAIN_MIN, PLAIN_MAX]: one Newton step from the
+// approximate reciprocal root. Before its last rounding the step is within
+// 1.5 sqrt(a) e^2 of the root for an approximation off by e; that this never
+// crosses a rounding boundary with this GPU's approximation was checked
+// against sqrtf for every float of the range (tests/test_gpu_plain_math.py).
+__device__ inline float sqrt_plain(float a) {
+    const float y = rsqrt_rough(a);
+    const float g = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-g, g, a), __fmul_rn(0.5f, y), g);
+}
+
+// RN(1 / b) for b in the plain range: one Newton step, checked in the same
+// way against __frcp_rn for every float of the range.
+__device__ inline float reciprocal_plain(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+
+// RN(a / b) from y = RN(1 / b), for |a| and b in [PLAIN_MIN, PLAIN_MAX]
+// (a = +0 too): the division by a correctly rounded reciprocal of
+// P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34 (1990). The first correction
+// makes q faithful, so the second residual a - b q is exact and the last FMA
+// rounds a / b + d with |d| <= b 2^-49 (b scaled to [1, 2)), below the
+// distance 2^-47 / b that a quotient of 24-bit numbers keeps from every
+// rounding boundary.
+__device__ inline float div_plain(float a, float b, float y) {
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+__device__ inline float min3_abs(float x, float y, float z) { return fminf(fminf(fabsf(x), fabsf(y)), fabsf(z)); }
+#endif
+
 // f32 arc cosine with one fixed rounding sequence, so that every build of
 // the relaxation (these kernels and the CPU oracle) rounds it identically.
 // The reference calls the backend's acos (kernels.rs:1211), whose last bits
@@ -72,6 +125,25 @@ __host__ __device__ inline float acos_f32(float x) {
     if (x > 0.0f) return 2.0f * r;
     return 2.0f * (pio2_hi - (r - pio2_lo));
 }
+
+#ifdef __CUDACC__
+// acos_f32 with the plain square root (its argument is 0 or at least 2^-25):
+// the same bits.
+__device__ inline float acos_plain(float x) {
+    const float pio2_hi = 1.57079637050628662109375f;
+    const float pio2_lo = -4.371138828673793e-08f;
+    const float ax = fabsf(x);
+    const bool middle = ax <= 0.5f;
+    const float z = middle ? x * x : 0.5f * (1.0f - ax);
+    const float s = middle ? x : z > 0.0f ? sqrt_plain(z) : 0.0f;
+    const float p = ((((0.03381037712097168f * z + 0.01707467809319496f) * z + 0.031116951256990433f) * z +
+                      0.04459794610738754f) * z + 0.07500099390745163f) * z + 0.1666666567325592f;
+    const float r = s + s * z * p;
+    if (!middle && x > 0.0f) return 2.0f * r;
+    const float t = pio2_hi - (r - pio2_lo);
+    return middle ? t : 2.0f * t;
+}
+#endif
 
 // proxy_cell (cell_list.rs:34-79) for a one-piece segment: the cell of its midpoint.
 __device__ inline uint32_t proxy_cell(float px, float py, float pz, float qx, float qy, float qz,

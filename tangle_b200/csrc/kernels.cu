@@ -1234,7 +1234,7 @@ __device__ inline bool curvature_triplet_test(const float4 *P, const float4 *St,
     float vx = pn.x - pc.x, vy = pn.y - pc.y, vz = pn.z - pc.z;
     const float uu = ux * ux + uy * uy + uz * uz;
     const float vv = vx * vx + vy * vy + vz * vz;
-    if (uu > 1.0e-12f && vv > 1.0e-12f) {  // the rough rejection of lanes_test, below
+    if (uu > 1.0e-12f && vv > 1.0e-12f) {  // the rough rejection of certainly_straight, below
         const float ru = rsqrtf(uu), rv = rsqrtf(vv);
         const float rough_half = 0.25f * maximum_curvature * (uu * ru + vv * rv);
         const float rough_limit = 1.0f - 2.0f * rough_half * rough_half;
@@ -1558,7 +1558,11 @@ __global__ void __launch_bounds__(256) fiber_kernel(WorldDev w, StepParams sp) {
 
 // ------------------------------------------------------ fiber update, lane per fiber
 
-constexpr int LANES_KMAX = 8;  // vertices per lane in the cooperative passes: fibers <= 256
+// Triplets per lane in the curvature sweeps: a strip's vertices (two more
+// than its triplets) and its triplets are bits of one word, and strips have
+// an odd length.
+constexpr int STRIP_MAX = 29;
+constexpr int STRIP_MIN = 5;
 
 // Shared-memory vertex record of the lane-per-fiber update: xyz, and w =
 // the vertex's curvature limit with the sign bit set when it is pinned
@@ -1566,85 +1570,407 @@ constexpr int LANES_KMAX = 8;  // vertices per lane in the cooperative passes: f
 __device__ inline bool lanes_pinned(float4 p) { return signbit(p.w); }
 __device__ inline float lanes_limit(float4 p) { return fabsf(p.w); }
 
-// project_curvature_triplet_in_place (kernels.rs:1165-1322) for triplet
-// (t, t+1, t+2) of a staged fiber, split into the test (does the projection
-// move anything?) and the move, so that a lane group can test several
-// triplets at once and apply only the first that acts. A cheap test first
-// rules out triplets that certainly satisfy their limit, before any IEEE
-// square root or division: edge lengths and the cosine from rsqrtf (2 ulp).
-// The rough limit cosine is within 2e-6 of the exact path's (whose lengths
-// are correctly rounded square roots) wherever the exact path can act, and
-// the rough cosine within 1e-6 of its cosine, so a 1e-5 margin never skips a
-// triplet the exact computation would project; the exact path that follows
-// is the reference's, operation for operation.
-__device__ inline bool lanes_test(const float4 *P, int t, float stiffness, float safety_margin, Triplet &tr) {
-    const float4 pp = P[t], pc = P[t + 1], pn = P[t + 2];
-    const float maximum_curvature = lanes_limit(pc) * (1.0f - safety_margin);
-    if (!(maximum_curvature > 0.0f)) return false;
-    const float ux = pc.x - pp.x, uy = pc.y - pp.y, uz = pc.z - pp.z;
-    const float vx = pn.x - pc.x, vy = pn.y - pc.y, vz = pn.z - pc.z;
-    const float uu = ux * ux + uy * uy + uz * uz;
-    const float vv = vx * vx + vy * vy + vz * vz;
-    if (uu > 1.0e-12f && vv > 1.0e-12f) {
-        const float ru = rsqrtf(uu), rv = rsqrtf(vv);
-        const float rough_half = 0.25f * maximum_curvature * (uu * ru + vv * rv);
-        const float rough_limit = 1.0f - 2.0f * rough_half * rough_half;
-        if ((ux * vx + uy * vy + uz * vz) * (ru * rv) > rough_limit + 1.0e-5f) return false;
+// Whether triplet (prev, center, next) certainly satisfies its limit, before
+// any IEEE square root or division: edge lengths and the cosine from the
+// approximate reciprocal square root (within 2 ulp). The rough limit cosine is within 2e-6 of the exact path's (whose
+// lengths are correctly rounded square roots) wherever the exact path can
+// act, and the rough cosine within 1e-6 of its cosine, so a 1e-5 margin never
+// skips a triplet the exact computation would project. uu, vv: squared edge
+// lengths; ru, rv: their reciprocal roots; dot: u . v.
+__device__ inline bool certainly_straight(float maximum_curvature, float uu, float vv, float ru, float rv, float dot) {
+    if (!(maximum_curvature > 0.0f)) return true;
+    if (!(uu > 1.0e-12f && vv > 1.0e-12f)) return false;
+    const float rough_half = 0.25f * maximum_curvature * (uu * ru + vv * rv);
+    const float rough_limit = 1.0f - 2.0f * rough_half * rough_half;
+    return dot * (ru * rv) > rough_limit + 1.0e-5f;
+}
+
+// Wall reactions of the vertices a strip's walk carries (FM only): a running
+// xyz per carried vertex, loaded from the fiber's reactions at the vertex's
+// first clamp of the pass.
+struct CarriedReaction {
+    float4 value;
+    bool held;
+};
+
+// The vertex that the sweep moved from `old` to `p`, kept inside the walls;
+// what the walls take from the move goes to its reaction (kernels.rs:
+// 1277-1305).
+template <bool FM>
+__device__ inline void keep_inside(float4 &p, float extent, const Grid &g, const float4 *R, int vertex, CarriedReaction &c) {
+    float moved[3] = {p.x, p.y, p.z}, kept[3];
+#pragma unroll
+    for (int axis = 0; axis < 3; ++axis) kept[axis] = wall_clamp(moved[axis], extent, axis, g);
+    p.x = kept[0], p.y = kept[1], p.z = kept[2];
+    if (FM && R != nullptr && !(kept[0] == moved[0] && kept[1] == moved[1] && kept[2] == moved[2])) {
+        if (!c.held) {
+            c.value = R[vertex];
+            c.held = true;
+        }
+        if (!(kept[0] == moved[0])) c.value.x += moved[0] - kept[0];
+        if (!(kept[1] == moved[1])) c.value.y += moved[1] - kept[1];
+        if (!(kept[2] == moved[2])) c.value.z += moved[2] - kept[2];
     }
-    const float first_length = sqrtf(uu);
-    const float second_length = sqrtf(vv);
-    if (!(first_length > 1.0e-7f && second_length > 1.0e-7f)) return false;
-    const float sine_half = 0.25f * maximum_curvature * (first_length + second_length);
+}
+
+// The gradients and the scale of a triplet's projection for edges e and f in
+// the pass's direction (kernels.rs:1165-1275): false when it moves nothing.
+struct Projection {
+    float ex, ey, ez, fx, fy, fz;  // gradients at the first and the last vertex
+    float scale;
+};
+
+// With the general operators, for operands outside the plain range.
+__device__ __noinline__ bool projection_general(Projection &t, float maximum_curvature, float stiffness, float w0, float w1,
+                                                float w2, bool forward) {
+    const float first = sqrtf(t.ex * t.ex + t.ey * t.ey + t.ez * t.ez);
+    const float second = sqrtf(t.fx * t.fx + t.fy * t.fy + t.fz * t.fz);
+    if (!(first > 1.0e-7f && second > 1.0e-7f)) return false;
+    const float ux = t.ex / first, uy = t.ey / first, uz = t.ez / first;
+    const float vx = t.fx / second, vy = t.fy / second, vz = t.fz / second;
+    const float cosine = clampf(ux * vx + uy * vy + uz * vz, -1.0f, 1.0f);
+    const float sine_half = 0.25f * maximum_curvature * (first + second);
     if (!(sine_half < 1.0f)) return false;
     const float minimum_cosine = 1.0f - 2.0f * sine_half * sine_half;
-    const float unx = ux / first_length, uny = uy / first_length, unz = uz / first_length;
-    const float vnx = vx / second_length, vny = vy / second_length, vnz = vz / second_length;
-    const float cosine = clampf(unx * vnx + uny * vny + unz * vnz, -1.0f, 1.0f);
     float violation = minimum_cosine - cosine;
     const float sine = sqrtf(fmaxf(1.0f - cosine * cosine, 0.0f));
     if (violation > 0.0f && sine > 1.0e-3f) violation = (acos_f32(cosine) - acos_f32(minimum_cosine)) * sine;
     if (!(violation > 0.0f)) return false;
-    tr.gux = (vnx - cosine * unx) / first_length;
-    tr.guy = (vny - cosine * uny) / first_length;
-    tr.guz = (vnz - cosine * unz) / first_length;
-    tr.gvx = (unx - cosine * vnx) / second_length;
-    tr.gvy = (uny - cosine * vny) / second_length;
-    tr.gvz = (unz - cosine * vnz) / second_length;
-    tr.cgx = tr.gux - tr.gvx;
-    tr.cgy = tr.guy - tr.gvy;
-    tr.cgz = tr.guz - tr.gvz;
-    tr.pw = lanes_pinned(pp) ? 0.0f : 1.0f;
-    tr.cw = lanes_pinned(pc) ? 0.0f : 1.0f;
-    tr.nw = lanes_pinned(pn) ? 0.0f : 1.0f;
-    const float denominator = tr.pw * (tr.gux * tr.gux + tr.guy * tr.guy + tr.guz * tr.guz) +
-                              tr.cw * (tr.cgx * tr.cgx + tr.cgy * tr.cgy + tr.cgz * tr.cgz) +
-                              tr.nw * (tr.gvx * tr.gvx + tr.gvy * tr.gvy + tr.gvz * tr.gvz);
+    t.ex = (vx - cosine * ux) / first;
+    t.ey = (vy - cosine * uy) / first;
+    t.ez = (vz - cosine * uz) / first;
+    t.fx = (ux - cosine * vx) / second;
+    t.fy = (uy - cosine * vy) / second;
+    t.fz = (uz - cosine * vz) / second;
+    const float cx = t.ex - t.fx, cy = t.ey - t.fy, cz = t.ez - t.fz;
+    const float a = w0 * (t.ex * t.ex + t.ey * t.ey + t.ez * t.ez), c = w2 * (t.fx * t.fx + t.fy * t.fy + t.fz * t.fz);
+    const float b = w1 * (cx * cx + cy * cy + cz * cz);
+    const float denominator = (forward ? a : c) + b + (forward ? c : a);
     if (!(denominator > 1.0e-12f)) return false;
-    tr.scale = stiffness * violation / denominator;
-    return tr.pw > 0.0f || tr.cw > 0.0f || tr.nw > 0.0f;
+    t.scale = stiffness * violation / denominator;
+    return true;
 }
 
-__device__ inline void lanes_apply(float4 *P, int t, const Triplet &tr, float extent, const Grid &g, float4 *R) {
-    const float4 pp = P[t], pc = P[t + 1], pn = P[t + 2];
-    float4 a = pp, b = pc, c = pn;
-    if (tr.pw > 0.0f) {
-        a.x = wall_clamp_r(pp.x - tr.pw * tr.scale * tr.gux, extent, 0, g, R, t);
-        a.y = wall_clamp_r(pp.y - tr.pw * tr.scale * tr.guy, extent, 1, g, R, t);
-        a.z = wall_clamp_r(pp.z - tr.pw * tr.scale * tr.guz, extent, 2, g, R, t);
+// project_curvature_triplet_in_place (kernels.rs:1165-1322) on three vertices
+// in the pass's direction that the cheap test did not rule out: true when it
+// moves them. Every operation rounds as the reference's does. Backward, the
+// reference's edges are the negatives of these, swapped; its unit vectors,
+// cosine, gradients and moves are then these, negated in pairs, so only the
+// denominator's order of summation differs. Nothing before the last test has
+// an effect, and nearly all triplets that come here act, so the two long
+// chains (the arc cosines; the gradients and their denominator) run beside
+// each other without a branch.
+template <bool FM>
+__device__ inline bool project_triplet(float4 &q0, float4 &q1, float4 &q2, bool forward, float stiffness,
+                                       float safety_margin, float extent, const Grid &g, bool walls, const float4 *R,
+                                       int v0, int v1, int v2, CarriedReaction &c0, CarriedReaction &c1,
+                                       CarriedReaction &c2) {
+    const float maximum_curvature = lanes_limit(q1) * (1.0f - safety_margin);
+    const float w0 = lanes_pinned(q0) ? 0.0f : 1.0f, w1 = lanes_pinned(q1) ? 0.0f : 1.0f, w2 = lanes_pinned(q2) ? 0.0f : 1.0f;
+    Projection t;
+    t.ex = q1.x - q0.x, t.ey = q1.y - q0.y, t.ez = q1.z - q0.z;
+    t.fx = q2.x - q1.x, t.fy = q2.y - q1.y, t.fz = q2.z - q1.z;
+    const float ee = t.ex * t.ex + t.ey * t.ey + t.ez * t.ez;
+    const float ff = t.fx * t.fx + t.fy * t.fy + t.fz * t.fz;
+    const float first = sqrt_plain(ee), second = sqrt_plain(ff);
+    const float first_inverse = reciprocal_plain(first), second_inverse = reciprocal_plain(second);
+    const float ux = div_plain(t.ex, first, first_inverse), uy = div_plain(t.ey, first, first_inverse),
+                uz = div_plain(t.ez, first, first_inverse);
+    const float vx = div_plain(t.fx, second, second_inverse), vy = div_plain(t.fy, second, second_inverse),
+                vz = div_plain(t.fz, second, second_inverse);
+    const float cosine = clampf(ux * vx + uy * vy + uz * vz, -1.0f, 1.0f);
+    const float nex = vx - cosine * ux, ney = vy - cosine * uy, nez = vz - cosine * uz;
+    const float nfx = ux - cosine * vx, nfy = uy - cosine * vy, nfz = uz - cosine * vz;
+    // No numerator is larger than its edge, or than 2; the smallest decides.
+    const bool plain = fminf(fminf(min3_abs(t.ex, t.ey, t.ez), min3_abs(t.fx, t.fy, t.fz)),
+                             fminf(min3_abs(nex, ney, nez), min3_abs(nfx, nfy, nfz))) >= PLAIN_MIN &&
+                       fminf(ee, ff) >= PLAIN_MIN && fmaxf(ee, ff) <= PLAIN_MAX;
+    bool acts;
+    if (plain) {
+        t.ex = div_plain(nex, first, first_inverse);
+        t.ey = div_plain(ney, first, first_inverse);
+        t.ez = div_plain(nez, first, first_inverse);
+        t.fx = div_plain(nfx, second, second_inverse);
+        t.fy = div_plain(nfy, second, second_inverse);
+        t.fz = div_plain(nfz, second, second_inverse);
+        const float cx = t.ex - t.fx, cy = t.ey - t.fy, cz = t.ez - t.fz;
+        const float a = w0 * (t.ex * t.ex + t.ey * t.ey + t.ez * t.ez), c = w2 * (t.fx * t.fx + t.fy * t.fy + t.fz * t.fz);
+        const float b = w1 * (cx * cx + cy * cy + cz * cz);
+        const float denominator = (forward ? a : c) + b + (forward ? c : a);
+        const float sine_half = 0.25f * maximum_curvature * (first + second);
+        const float minimum_cosine = 1.0f - 2.0f * sine_half * sine_half;
+        float violation = minimum_cosine - cosine;
+        const float sine2 = fmaxf(1.0f - cosine * cosine, 0.0f);  // 0 or at least 2^-24
+        const float sine = sine2 > 0.0f ? sqrt_plain(sine2) : 0.0f;
+        const float angle = acos_plain(cosine) - acos_plain(fmaxf(minimum_cosine, -1.0f));
+        if (violation > 0.0f && sine > 1.0e-3f) violation = angle * sine;
+        acts = first > 1.0e-7f && second > 1.0e-7f && sine_half < 1.0f && violation > 0.0f && denominator > 1.0e-12f;
+        t.scale = stiffness * violation / denominator;
+    } else {
+        acts = projection_general(t, maximum_curvature, stiffness, w0, w1, w2, forward);
     }
-    if (tr.cw > 0.0f) {
-        b.x = wall_clamp_r(pc.x + tr.cw * tr.scale * tr.cgx, extent, 0, g, R, t + 1);
-        b.y = wall_clamp_r(pc.y + tr.cw * tr.scale * tr.cgy, extent, 1, g, R, t + 1);
-        b.z = wall_clamp_r(pc.z + tr.cw * tr.scale * tr.cgz, extent, 2, g, R, t + 1);
+    if (!acts || !(w0 > 0.0f || w1 > 0.0f || w2 > 0.0f)) return false;
+    if (w0 > 0.0f) {
+        q0.x -= t.scale * t.ex, q0.y -= t.scale * t.ey, q0.z -= t.scale * t.ez;
+        if (walls) keep_inside<FM>(q0, extent, g, R, v0, c0);
     }
-    if (tr.nw > 0.0f) {
-        c.x = wall_clamp_r(pn.x + tr.nw * tr.scale * tr.gvx, extent, 0, g, R, t + 2);
-        c.y = wall_clamp_r(pn.y + tr.nw * tr.scale * tr.gvy, extent, 1, g, R, t + 2);
-        c.z = wall_clamp_r(pn.z + tr.nw * tr.scale * tr.gvz, extent, 2, g, R, t + 2);
+    if (w1 > 0.0f) {
+        q1.x += t.scale * (t.ex - t.fx), q1.y += t.scale * (t.ey - t.fy), q1.z += t.scale * (t.ez - t.fz);
+        if (walls) keep_inside<FM>(q1, extent, g, R, v1, c1);
     }
-    P[t] = a;
-    P[t + 1] = b;
-    P[t + 2] = c;
+    if (w2 > 0.0f) {
+        q2.x += t.scale * t.fx, q2.y += t.scale * t.fy, q2.z += t.scale * t.fz;
+        if (walls) keep_inside<FM>(q2, extent, g, R, v2, c2);
+    }
+    return true;
+}
+
+// project_fiber_curvature_in_place (kernels.rs:1324-1415): the forward and
+// backward Gauss-Seidel sweeps of 32 / G fibers, G lanes per fiber, the
+// warp's fibers in step. X: the fiber's staged vertices (odd strides, so
+// that strided reads spread over the banks), Y: room for as many, T: its
+// triplets (at most 29 G; 0 or less: no fiber). Returns the rounds taken.
+//
+// A pass is a recurrence along the fiber: triplet k (counted in the pass's
+// direction) reads vertices k, k + 1, k + 2, of which only k and k + 1 can
+// have moved in this pass, and only by triplets k - 1 and k - 2. So the pass
+// is cut into G strips, one lane each, and every lane walks its strip at
+// once on the assumption that the two triplets before it do not act: most
+// triplets do not (6 % of them on a relaxed packing, 10 to 30 % on a fresh
+// one), and a strip between two idle ones is on its own. A lane carries the
+// two moved vertices in registers, reads the third from X, which stays as
+// the pass found it, and writes finished vertices that moved to Y. Then each
+// lane passes its last two vertices on; where they moved, the next lane
+// walks again from them, until it meets a point that its earlier walk passed
+// with nothing moved (the rest stands) or hands on in turn. Lane l's result
+// is final after at most l + 1 walks, so this ends, and every triplet has
+// then been computed from exactly the inputs that the serial pass gives it.
+//
+// Within a strip a lane only visits triplets that may act: those that the
+// cheap test on X does not rule out (a sliding scan, one vertex load and one
+// edge per triplet) and the two after each acting one. A pass that moves
+// nothing ends its fiber's sweeps (every later pass would test the same
+// positions).
+//
+// What bounds it: the projection's chain (about 290 instructions, 730 cycles
+// on a lone warp) times the longest run of triplets that wait for each other,
+// and instruction issue where the chip is full. The former sweep applied one
+// acting triplet of 8 tested ones per round and fiber: 25-42 rounds per
+// update on 31-vertex fibers, 130-150 on the mid-size specimen's and 465 on
+// 180-vertex ply fibers; strips take 6-20, 28-39 and 145-185. Update stage
+// before and after: 40 fibers of 31 vertices 107 -> 62 us per launch, 2,000
+// of 108 380 -> 122 us, 20,000 of 108 700 -> 481 us, 886 of 66 and 180
+// between walls 1,382 -> 412 us, 357-vertex fibers 2,373 -> 507 us (there
+// from one warp per fiber that tested 32 triplets a round).
+template <int G, bool FM>
+__device__ inline uint32_t sweep_curvature(float4 *X, float4 *Y, int T, const StepParams &sp, float extent, const Grid &g,
+                                           float4 *R, float4 *R_next) {
+    const int lane = threadIdx.x & 31, group = lane / G, gl = lane % G;
+    const uint32_t gmask = G == 32 ? FULL : ((1u << G) - 1u) << (group * G);
+    const int L = max((T + G - 1) / G, STRIP_MIN) | 1;
+    const int a = min(gl * L, max(T, 0)), b = min(a + L, max(T, 0));
+    const float stiffness = sp.curvature_limit_stiffness, safety = sp.curvature_limit_safety_margin;
+    const bool walls = !(g.periodic[0] && g.periodic[1] && g.periodic[2]);
+    bool done = T <= 0;
+    uint32_t rounds = 0;
+    for (uint32_t pass = 0; pass < 2 * sp.curvature_cleanup_sweeps; ++pass) {
+        if (!__any_sync(FULL, !done)) break;
+        const bool forward = (pass & 1u) == 0u;
+        // Vertex k of the pass's direction.
+        const int origin = forward ? 0 : T + 1, sign = forward ? 1 : -1;
+        const auto at = [&](int k) { return origin + sign * k; };
+        // The strip's triplets that may act on the positions as they are.
+        uint32_t may = 0;
+        if (!done && a < b) {
+            float4 q1 = X[at(a)];
+            float4 q2 = X[at(a + 1)];
+            float ex = q2.x - q1.x, ey = q2.y - q1.y, ez = q2.z - q1.z;
+            float uu = ex * ex + ey * ey + ez * ez, ru = rsqrt_rough(uu);
+#pragma unroll 4
+            for (int k = a; k < b; ++k) {
+                q1 = q2;
+                q2 = X[at(k + 2)];
+                const float fx = q2.x - q1.x, fy = q2.y - q1.y, fz = q2.z - q1.z;
+                const float vv = fx * fx + fy * fy + fz * fz, rv = rsqrt_rough(vv);
+                if (!certainly_straight(lanes_limit(q1) * (1.0f - safety), uu, vv, ru, rv, ex * fx + ey * fy + ez * fz))
+                    may |= 1u << (k - a);
+                ex = fx, ey = fy, ez = fz, uu = vv, ru = rv;
+            }
+        }
+        // The walks. acted / moved / reacted: bits from the strip's first
+        // triplet / vertex; came, left: how many of the two vertices handed
+        // in / out had moved (2: both, 1: the first).
+        uint32_t acted = 0, moved = 0, reacted = 0, old_acted = 0, old_moved = 0, old_reacted = 0;
+        int came = 0, old_came = 0, left = 0, k = a;
+        int dirty = 0;  // of triplet k's vertices, the first so many have moved
+        bool again = false;  // a repeated walk
+        bool changed = false;
+        float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q1 = q0, q2 = q0, q3 = q0, q4 = q0;
+        CarriedReaction c0{}, c1{}, c2{};
+        // Loads the first triplet that may act at or after k, with nothing
+        // moved before it (false: there is none).
+        const auto load = [&]() {
+            const uint32_t rest = k < b ? may >> (k - a) : 0u;
+            if (rest == 0) return false;
+            k += __ffs(rest) - 1;
+            q0 = X[at(k)];
+            q1 = X[at(k + 1)];
+            q2 = X[at(k + 2)];
+            dirty = 0;
+            if (FM) c0.held = c1.held = c2.held = false;
+            return true;
+        };
+        // A vertex is finished: kept where it moved.
+        const auto keep = [&](bool finished, int vertex, const float4 &q, const CarriedReaction &c) {
+            if (finished) {
+                Y[at(vertex)] = q;
+                moved |= 1u << (vertex - a);
+                if (FM && c.held) {
+                    R_next[at(vertex)] = c.value;
+                    reacted |= 1u << (vertex - a);
+                }
+            }
+        };
+        bool walking = load();   // a triplet to project is loaded
+        bool stepping = false;   // the walk steps on from triplet k
+        for (;;) {
+            for (;;) {
+                if (stepping) {
+                    // The next two triplets see moved vertices; both are
+                    // tested at once (the second as if the first were idle).
+                    stepping = false;
+                    const int d1 = dirty - 1, d2 = dirty - 2, rest = b - (k + 1);
+                    const float ex = q2.x - q1.x, ey = q2.y - q1.y, ez = q2.z - q1.z;
+                    const float fx = q3.x - q2.x, fy = q3.y - q2.y, fz = q3.z - q2.z;
+                    const float gx = q4.x - q3.x, gy = q4.y - q3.y, gz = q4.z - q3.z;
+                    const float ee = ex * ex + ey * ey + ez * ez, ff = fx * fx + fy * fy + fz * fz,
+                                gg = gx * gx + gy * gy + gz * gz;
+                    const float re = rsqrt_rough(ee), rf = rsqrt_rough(ff), rg = rsqrt_rough(gg);
+                    const bool next1 = d1 > 0 && rest > 0 &&
+                                       !certainly_straight(lanes_limit(q2) * (1.0f - safety), ee, ff, re, rf,
+                                                           ex * fx + ey * fy + ez * fz);
+                    const bool next2 = !next1 && d2 > 0 && rest > 1 &&
+                                       !certainly_straight(lanes_limit(q3) * (1.0f - safety), ff, gg, rf, rg,
+                                                           fx * gx + fy * gy + fz * gz);
+                    // The strip ends with moved vertices.
+                    const bool end = !next1 && !next2 && ((d1 > 0 && rest == 0) || (d2 > 0 && rest == 1));
+                    const bool hand = end && b < T;
+                    keep(d1 > 0 && !next1 && !(hand && rest == 0), k + 1, q1, c1);
+                    keep(d2 > 0 && !next1 && !next2 && !hand, k + 2, q2, c2);
+                    if (next1 || (hand && rest == 0)) {
+                        q0 = q1, q1 = q2, q2 = q3;
+                        if (FM) {
+                            c0 = c1, c1 = c2;
+                            c2.held = false;
+                        }
+                        k += 1;
+                        dirty = d1;
+                    } else if (next2 || hand) {
+                        q0 = q2, q1 = q3, q2 = q4;
+                        if (FM) {
+                            c0 = c2;
+                            c1.held = c2.held = false;
+                        }
+                        k += 2;
+                        dirty = d2;
+                    }
+                    walking = next1 || next2;
+                    if (end) {
+                        changed = hand;
+                        left = dirty;
+                    } else if (!walking) {
+                        k += 1 + max(d1, 0);
+                        walking = load();
+                        const int r = k - a;
+                        const uint32_t before = r >= 2 ? 3u << (r - 2) : r == 1 ? 1u : 0u;
+                        if (!walking) {
+                            changed = again && left > 0;
+                            left = 0;
+                        } else if (again && (old_acted & before) == 0 && r >= old_came) {
+                            // The earlier walk came here with nothing moved
+                            // too: from here on it stands.
+                            acted |= old_acted >> r << r;
+                            moved |= old_moved >> r << r;
+                            reacted |= old_reacted >> r << r;
+                            walking = false;
+                            changed = false;
+                        }
+                    }
+                }
+                const uint32_t walkers = __ballot_sync(FULL, walking);
+                if (walkers == 0) break;
+                if (walkers & gmask) ++rounds;
+                if (walking) {
+                    q3 = X[at(min(k + 3, T + 1))];
+                    q4 = X[at(min(k + 4, T + 1))];
+                    if (project_triplet<FM>(q0, q1, q2, forward, stiffness, safety, extent, g, walls, R, at(k), at(k + 1),
+                                            at(k + 2), c0, c1, c2)) {
+                        acted |= 1u << (k - a);
+                        dirty = 3;
+                    }
+                    keep(dirty > 0, k, q0, c0);
+                    walking = false;
+                    stepping = true;
+                }
+            }
+            if (!__any_sync(FULL, changed)) break;
+            // Hand the last two vertices on to the lanes whose incoming ones
+            // are others than they walked from.
+            const bool next = __shfl_up_sync(FULL, changed ? 1 : 0, 1, G) != 0 && gl > 0 && a < b;
+            const int arriving = __shfl_up_sync(FULL, left, 1, G);
+            const float hx0 = __shfl_up_sync(FULL, q0.x, 1, G), hy0 = __shfl_up_sync(FULL, q0.y, 1, G),
+                        hz0 = __shfl_up_sync(FULL, q0.z, 1, G), hx1 = __shfl_up_sync(FULL, q1.x, 1, G),
+                        hy1 = __shfl_up_sync(FULL, q1.y, 1, G), hz1 = __shfl_up_sync(FULL, q1.z, 1, G);
+            CarriedReaction h0{}, h1{};
+            if (FM) {
+                h0.held = __shfl_up_sync(FULL, c0.held ? 1 : 0, 1, G) != 0;
+                h1.held = __shfl_up_sync(FULL, c1.held ? 1 : 0, 1, G) != 0;
+                h0.value.x = __shfl_up_sync(FULL, c0.value.x, 1, G);
+                h0.value.y = __shfl_up_sync(FULL, c0.value.y, 1, G);
+                h0.value.z = __shfl_up_sync(FULL, c0.value.z, 1, G);
+                h1.value.x = __shfl_up_sync(FULL, c1.value.x, 1, G);
+                h1.value.y = __shfl_up_sync(FULL, c1.value.y, 1, G);
+                h1.value.z = __shfl_up_sync(FULL, c1.value.z, 1, G);
+            }
+            changed = false;
+            if (next) {
+                old_acted = acted, old_moved = moved, old_reacted = reacted, old_came = came;
+                acted = moved = reacted = 0;
+                again = true;
+                came = arriving;
+                // As if stepping on from the triplet before the strip.
+                k = a - 1;
+                dirty = arriving + 1;
+                if (arriving > 0) {
+                    q1 = X[at(a)];
+                    q2 = X[at(a + 1)];
+                    q3 = X[at(a + 2)];
+                    q4 = X[at(min(a + 3, T + 1))];
+                    q1.x = hx0, q1.y = hy0, q1.z = hz0;
+                    q2.x = hx1, q2.y = hy1, q2.z = hz1;
+                    if (FM) c1 = h0, c2 = h1;
+                }
+                stepping = true;
+            }
+        }
+        __syncwarp();
+        const bool acts = acted != 0;
+        // The finished vertices that moved become the next pass's positions.
+        while (moved) {
+            const int v = at(a + __ffs(moved) - 1);
+            moved &= moved - 1u;
+            X[v] = Y[v];
+        }
+        if (FM)
+            while (reacted) {
+                const int v = at(a + __ffs(reacted) - 1);
+                reacted &= reacted - 1u;
+                R[v] = R_next[v];
+            }
+        __syncwarp();
+        if ((__ballot_sync(FULL, acts) & gmask) == 0) done = true;
+    }
+    return rounds;
 }
 
 // Order of the grouped-lane update's fibers. A warp's lane groups step
@@ -1779,25 +2105,22 @@ __global__ void __launch_bounds__(ORDER_THREADS) order_by_rounds_kernel(WorldDev
     }
 }
 
-// Everything after the gate for 32/LPF fibers per warp (fibers of at most
-// 256 vertices), LPF lanes per fiber in the curvature sweeps. The warp stages
-// the fibers in shared memory and runs the internal stretch/bend passes
-// (kernels.rs:1027-1163, :1417-1453) and the contact step (:1455-1537)
-// cooperatively, one fiber at a time. Then each group of LPF lanes runs
-// project_fiber_curvature_in_place (:1324-1415) on its fiber: the group tests
-// LPF consecutive triplets on the current positions; every triplet before
-// the first acting one is a no-op in the serial order, so applying that one
-// and resuming right after it reproduces the serial sweep exactly. Last the
-// warp writes the fibers back with the displacement check
-// (neighbor.rs:446-465) and the next gate's curvature and step maxima
-// (:925-980, :95-127).
+// Everything after the gate for 32/LPF fibers per warp, LPF lanes per fiber
+// in the curvature sweeps (fibers of at most LPF x STRIP_MAX + 2 vertices).
+// The warp stages the fibers in shared memory, two records per vertex, and
+// runs the internal stretch/bend passes (kernels.rs:1027-1163, :1417-1453)
+// from one to the other and the contact step (:1455-1537) cooperatively, one
+// fiber at a time. Then sweep_curvature runs project_fiber_curvature_in_place
+// (:1324-1415) on all of them. Last the warp writes the fibers back with the
+// displacement check (neighbor.rs:446-465) and the next gate's curvature and
+// step maxima (:925-980, :95-127).
 // In an arena (A) each fiber takes its specimen's grid and skin, fibers of
 // stopped specimens are skipped, and the maxima and flags go to each
 // fiber's specimen.
 // FM compiles in the formation work (wall reactions, layer and vertex
 // targets); without it the kernel carries none of it.
 template <int LPF, bool A = false, bool FM = false>
-__global__ void __launch_bounds__(128, 8) fiber_lanes_kernel(WorldDev w, StepParams sp, int stride) {
+__global__ void __launch_bounds__(128, A ? 6 : 4) fiber_lanes_kernel(WorldDev w, StepParams sp, int stride) {
     constexpr int FPW = 32 / LPF;  // fibers per warp
     if (w.ctl->control[0] == 0) return;
     extern __shared__ float4 lanes_smem_all[];
@@ -1805,9 +2128,14 @@ __global__ void __launch_bounds__(128, 8) fiber_lanes_kernel(WorldDev w, StepPar
     // only so that 32 warps fit on an SM (at most 32 blocks are resident).
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    float4 *const lanes_smem = lanes_smem_all + (size_t)wib * FPW * stride;
+    // The warp's fibers in one record array, and as much room again; the
+    // internal passes read one and write the other.
+    float4 *const lanes_smem = lanes_smem_all + (size_t)wib * 2 * FPW * stride;
+    float4 *const lanes_room = lanes_smem + (size_t)FPW * stride;
+    const bool swapped = (sp.constraint_iterations & 1u) != 0u;
+    float4 *const staged = swapped ? lanes_room : lanes_smem;  // after the internal passes
+    float4 *const room = swapped ? lanes_smem : lanes_room;
     const int group = lane / LPF, gl = lane % LPF;
-    const uint32_t gmask = LPF == 32 ? FULL : (((1u << LPF) - 1u) << (group * LPF));
     uint32_t smax = 0, cmax = 0;
     bool far = false;
     bool contact_far = false;
@@ -1838,80 +2166,66 @@ __global__ void __launch_bounds__(128, 8) fiber_lanes_kernel(WorldDev w, StepPar
             }
             __syncwarp();
             // find/apply_internal_corrections x constraint_iterations (Jacobi).
+            float4 *Q = lanes_room + (size_t)j * stride;
             for (uint32_t pass = 0; pass < sp.constraint_iterations; ++pass) {
-                float cxs[LANES_KMAX], cys[LANES_KMAX], czs[LANES_KMAX];
-#pragma unroll
-                for (int k = 0; k < LANES_KMAX; ++k) {
-                    const int i = lane + 32 * k;
-                    float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-                    if (i < n) {
-                        const float4 x = P[i];
-                        if (!lanes_pinned(x)) {
-                            if (i > 0) {
-                                float4 o = P[i - 1];
-                                float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
-                                float length = sqrtf(dx * dx + dy * dy + dz * dz);
-                                if (length > 1.0e-7f) {
-                                    float magnitude = 0.5f * sp.stretch_stiffness * (length - w.rest[s0 + i - 1]) / length;
-                                    cx += dx * magnitude;
-                                    cy += dy * magnitude;
-                                    cz += dz * magnitude;
-                                }
-                            }
-                            if (i + 1 < n) {
-                                float4 o = P[i + 1];
-                                float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
-                                float length = sqrtf(dx * dx + dy * dy + dz * dz);
-                                if (length > 1.0e-7f) {
-                                    float magnitude = 0.5f * sp.stretch_stiffness * (length - w.rest[s0 + i]) / length;
-                                    cx += dx * magnitude;
-                                    cy += dy * magnitude;
-                                    cz += dz * magnitude;
-                                }
-                            }
-                            if (i > 1) {
-                                float4 o = P[i - 2];
-                                float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
-                                float length = sqrtf(dx * dx + dy * dy + dz * dz);
-                                if (length > 1.0e-7f) {
-                                    float magnitude = 0.5f * sp.bend_stiffness * (length - w.vtx_static[v0 + i].y) / length;
-                                    cx += dx * magnitude;
-                                    cy += dy * magnitude;
-                                    cz += dz * magnitude;
-                                }
-                            }
-                            if (i + 2 < n) {
-                                float4 o = P[i + 2];
-                                float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
-                                float length = sqrtf(dx * dx + dy * dy + dz * dz);
-                                if (length > 1.0e-7f) {
-                                    float magnitude = 0.5f * sp.bend_stiffness * (length - w.vtx_static[v0 + i].z) / length;
-                                    cx += dx * magnitude;
-                                    cy += dy * magnitude;
-                                    cz += dz * magnitude;
-                                }
+                for (int i = lane; i < n; i += 32) {
+                    float4 x = P[i];
+                    if (!lanes_pinned(x)) {
+                        float cx = 0.0f, cy = 0.0f, cz = 0.0f;
+                        if (i > 0) {
+                            float4 o = P[i - 1];
+                            float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
+                            float length = sqrtf(dx * dx + dy * dy + dz * dz);
+                            if (length > 1.0e-7f) {
+                                float magnitude = 0.5f * sp.stretch_stiffness * (length - w.rest[s0 + i - 1]) / length;
+                                cx += dx * magnitude;
+                                cy += dy * magnitude;
+                                cz += dz * magnitude;
                             }
                         }
-                    }
-                    cxs[k] = cx;
-                    cys[k] = cy;
-                    czs[k] = cz;
-                }
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < LANES_KMAX; ++k) {
-                    const int i = lane + 32 * k;
-                    if (i < n) {
-                        float4 x = P[i];
-                        if (!lanes_pinned(x)) {
-                            x.x = wall_clamp_r(x.x + cxs[k], extent, 0, g, R, i);
-                            x.y = wall_clamp_r(x.y + cys[k], extent, 1, g, R, i);
-                            x.z = wall_clamp_r(x.z + czs[k], extent, 2, g, R, i);
-                            P[i] = x;
+                        if (i + 1 < n) {
+                            float4 o = P[i + 1];
+                            float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
+                            float length = sqrtf(dx * dx + dy * dy + dz * dz);
+                            if (length > 1.0e-7f) {
+                                float magnitude = 0.5f * sp.stretch_stiffness * (length - w.rest[s0 + i]) / length;
+                                cx += dx * magnitude;
+                                cy += dy * magnitude;
+                                cz += dz * magnitude;
+                            }
                         }
+                        if (i > 1) {
+                            float4 o = P[i - 2];
+                            float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
+                            float length = sqrtf(dx * dx + dy * dy + dz * dz);
+                            if (length > 1.0e-7f) {
+                                float magnitude = 0.5f * sp.bend_stiffness * (length - w.vtx_static[v0 + i].y) / length;
+                                cx += dx * magnitude;
+                                cy += dy * magnitude;
+                                cz += dz * magnitude;
+                            }
+                        }
+                        if (i + 2 < n) {
+                            float4 o = P[i + 2];
+                            float dx = o.x - x.x, dy = o.y - x.y, dz = o.z - x.z;
+                            float length = sqrtf(dx * dx + dy * dy + dz * dz);
+                            if (length > 1.0e-7f) {
+                                float magnitude = 0.5f * sp.bend_stiffness * (length - w.vtx_static[v0 + i].z) / length;
+                                cx += dx * magnitude;
+                                cy += dy * magnitude;
+                                cz += dz * magnitude;
+                            }
+                        }
+                        x.x = wall_clamp_r(x.x + cx, extent, 0, g, R, i);
+                        x.y = wall_clamp_r(x.y + cy, extent, 1, g, R, i);
+                        x.z = wall_clamp_r(x.z + cz, extent, 2, g, R, i);
                     }
+                    Q[i] = x;
                 }
                 __syncwarp();
+                float4 *const t = P;
+                P = Q;
+                Q = t;
             }
             // apply_contact_corrections (flexible).
             for (int i = lane; i < n; i += 32) {
@@ -1954,59 +2268,16 @@ __global__ void __launch_bounds__(128, 8) fiber_lanes_kernel(WorldDev w, StepPar
                 smax = 0;
             }
         }
-        // Curvature Gauss-Seidel, LPF lanes per fiber, forward then backward.
-        // The warp's groups step together: every round each unfinished group
-        // tests LPF triplets of its own fiber, one warp-wide ballot gives
-        // every group its bits, and each group applies its own first acting
-        // triplet. A group's sequence of tests and moves is exactly its
-        // serial sweep; stepping together only shares the instruction issue
-        // between the groups. A pass that moves nothing ends its group's
-        // sweeps (every later pass would test the same positions).
+        // Curvature Gauss-Seidel, LPF lanes per fiber.
         {
             const Grid &g = grid_of<A>(w, mine != TGL_NONE ? spec_of_fiber<A>(w, mine) : 0u);
-            const int last = mine != TGL_NONE ? (int)w.fiber_vspan[mine].y - 3 : -1;
+            const int triplets = mine != TGL_NONE ? (int)w.fiber_vspan[mine].y - 2 : 0;
             const float extent = mine != TGL_NONE ? w.seg_static[w.fiber_s0[mine]].x : 0.0f;
-            float4 *const R =
-                FM && mine != TGL_NONE && w.reaction != nullptr ? w.reaction + w.fiber_vspan[mine].x : nullptr;
-            float4 *P = lanes_smem + (size_t)group * stride;
-            bool done = mine == TGL_NONE || sp.curvature_cleanup_sweeps == 0;
-            bool forward = true, moved = false;
-            uint32_t sweep = 0, rounds = 0;
-            int t0 = 0;
-            while (__any_sync(FULL, !done)) {
-                rounds += done ? 0u : 1u;
-                Triplet tr;
-                const int t = forward ? t0 + gl : t0 - gl;
-                const bool act = !done && (forward ? t <= last : t >= 0) &&
-                                 lanes_test(P, t, sp.curvature_limit_stiffness, sp.curvature_limit_safety_margin, tr);
-                const uint32_t ballot = __ballot_sync(FULL, act);
-                const uint32_t bits = LPF == 32 ? ballot : (ballot >> (group * LPF)) & ((1u << LPF) - 1u);
-                if (!done) {
-                    if (bits) {
-                        const int first = __ffs(bits) - 1;
-                        if (gl == first) lanes_apply(P, t, tr, extent, g, R);
-                        moved = true;
-                        t0 = forward ? t0 + first + 1 : t0 - first - 1;
-                    } else {
-                        t0 = forward ? t0 + LPF : t0 - LPF;
-                    }
-                    if (forward ? t0 > last : t0 < 0) {  // the pass is over
-                        if (!moved) {
-                            done = true;
-                        } else if (forward) {
-                            forward = false;
-                            moved = false;
-                            t0 = last;
-                        } else {
-                            moved = false;
-                            forward = true;
-                            t0 = 0;
-                            done = ++sweep >= sp.curvature_cleanup_sweeps;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
+            const bool reacts = FM && mine != TGL_NONE && w.reaction != nullptr;
+            float4 *const R = reacts ? w.reaction + w.fiber_vspan[mine].x : nullptr;
+            float4 *const R_next = reacts ? w.reaction_next + w.fiber_vspan[mine].x : nullptr;
+            const uint32_t rounds = sweep_curvature<LPF, FM>(staged + (size_t)group * stride, room + (size_t)group * stride,
+                                                             triplets, sp, extent, g, R, R_next);
             // The rounds this fiber's sweeps took rank it for the next updates
             // (a fiber of a stopped specimen took none).
             if (!A && w.fiber_rounds != nullptr && mine != TGL_NONE && gl == 0) w.fiber_rounds[mine] = rounds;
@@ -2025,7 +2296,7 @@ __global__ void __launch_bounds__(128, 8) fiber_lanes_kernel(WorldDev w, StepPar
             const int n = (int)span.y;
             const uint32_t s0 = w.fiber_s0[f];
             const float radius = w.seg_static[s0].x;
-            float4 *P = lanes_smem + (size_t)j * stride;
+            float4 *P = staged + (size_t)j * stride;
             if (FM) formation_targets_staged(w, f, P, n, v0, lane);
             for (int i = lane; i < n; i += 32) {
                 const float4 x = P[i];
@@ -2331,17 +2602,24 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     lp.fiber_warps = warps;
     lp.fiber_smem = per_warp * warps;
     lp.fiber_blocks = grid_for(w.FA, warps, 1 << 20);
-    // Lane-per-fiber update for fibers of at most 32 * LANES_KMAX vertices:
-    // 32 fibers per warp, an odd float4 stride per fiber so that the lanes'
-    // same-index accesses spread over the banks.
+    // Grouped-lane update: an odd float4 stride per fiber so that the groups'
+    // same-index accesses spread over the banks. The lanes per fiber asked
+    // for are raised until a strip's triplets fit its word.
+    // By default a warp per fiber while all of those warps are resident at
+    // once (the sweeps' chains then take all the lanes there are), and a
+    // quarter warp where the chip is full without (four fibers share each
+    // round's instructions).
+    lp.lanes_per_fiber = w.FA <= (uint32_t)lp.num_sms * 16u ? 32 : 8;
     if (const char *env = std::getenv("TGL_LANES_PER_FIBER")) lp.lanes_per_fiber = std::atoi(env);
     if (lp.tune_lanes) lp.lanes_per_fiber = lp.tune_lanes;
     if (lp.lanes_per_fiber != 2 && lp.lanes_per_fiber != 4 && lp.lanes_per_fiber != 8 && lp.lanes_per_fiber != 32)
         lp.lanes_per_fiber = 8;
-    const int fpw = 32 / lp.lanes_per_fiber;
+    lp.strip_lanes = lp.lanes_per_fiber < 4 ? 4 : lp.lanes_per_fiber;
+    while (lp.strip_lanes < 32 && (int)w.max_fiber - 2 > lp.strip_lanes * STRIP_MAX) lp.strip_lanes *= 2;
+    const int fpw = 32 / lp.strip_lanes;
     lp.lanes_stride = (int)(w.max_fiber | 1u);
-    lp.lanes_smem = (size_t)fpw * lp.lanes_stride * sizeof(float4);
-    lp.fiber_lanes = w.max_fiber <= 32u * LANES_KMAX && lp.lanes_smem <= 200 * 1024;
+    lp.lanes_smem = (size_t)2 * fpw * lp.lanes_stride * sizeof(float4);
+    lp.fiber_lanes = (int)w.max_fiber - 2 <= 32 * STRIP_MAX && lp.lanes_smem <= 200 * 1024;
     // Warps per block: 4 where their staged fibers fit, so that 32 warps
     // (the register file at the kernel's 64 registers, and 8 blocks of 4
     // warps) are resident per SM instead of the 28 that one-warp blocks get
@@ -2381,15 +2659,15 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     if (lp.fiber_lanes) {
         const size_t smem = lp.lanes_smem * lp.lanes_wpb;
         const auto allow = [smem](auto kernel) { allow_dynamic_smem(kernel, smem); };
-        allow(fiber_lanes_kernel<2, false, false>);
+        allow(fiber_lanes_kernel<16, false, false>);
         allow(fiber_lanes_kernel<4, false, false>);
         allow(fiber_lanes_kernel<8, false, false>);
         allow(fiber_lanes_kernel<32, false, false>);
-        allow(fiber_lanes_kernel<2, true, false>);
+        allow(fiber_lanes_kernel<16, true, false>);
         allow(fiber_lanes_kernel<4, true, false>);
         allow(fiber_lanes_kernel<8, true, false>);
         allow(fiber_lanes_kernel<32, true, false>);
-        allow(fiber_lanes_kernel<2, false, true>);
+        allow(fiber_lanes_kernel<16, false, true>);
         allow(fiber_lanes_kernel<4, false, true>);
         allow(fiber_lanes_kernel<8, false, true>);
         allow(fiber_lanes_kernel<32, false, true>);
@@ -2526,9 +2804,9 @@ template <bool A, bool FM>
 static void enqueue_lanes(const WorldDev &w, const LaunchPlan &lp, const StepParams &sp, cudaStream_t st) {
     const dim3 grid(lp.lanes_blocks), block(32 * lp.lanes_wpb);
     const size_t smem = lp.lanes_smem * lp.lanes_wpb;
-    switch (lp.lanes_per_fiber) {
-        case 2: fiber_lanes_kernel<2, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
+    switch (lp.strip_lanes) {
         case 8: fiber_lanes_kernel<8, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
+        case 16: fiber_lanes_kernel<16, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
         case 32: fiber_lanes_kernel<32, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
         default: fiber_lanes_kernel<4, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
     }

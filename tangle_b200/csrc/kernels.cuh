@@ -109,6 +109,7 @@ struct WorldDev {
     // curvature cleanup): xyz per vertex, w unused; nullptr when no axis has
     // walls (every reaction is then zero).
     float4 *reaction;          // [V]
+    float4 *reaction_next;     // [V] of a sweep's vertices until its pass is over
     // Formation layer target (kernels.rs:538-581), applied at the end of
     // every update step while layer_target is set.
     const uint32_t *fiber_layer; // [F] layer of each fiber, TGL_NONE = none
@@ -224,8 +225,9 @@ struct LaunchPlan {
     int fiber_warps;        // fibers per block of the update kernel
     int fiber_blocks;
     size_t fiber_smem;
-    bool fiber_lanes;       // grouped-lane update (fibers of at most 256 vertices)
-    int lanes_per_fiber;    // lanes per fiber in its curvature sweeps (2, 4, 8 or 32)
+    bool fiber_lanes;       // grouped-lane update (fibers of at most 930 vertices)
+    int lanes_per_fiber;    // lanes per fiber in its curvature sweeps asked for (2, 4, 8 or 32)
+    int strip_lanes;        // and taken: at least 4, and enough for the longest fiber
     int lanes_stride;
     size_t lanes_smem;      // staged fibers of one warp
     int lanes_wpb;          // warps per block (1, 2 or 4)

@@ -877,7 +877,7 @@ int build_world(std::vector<HostSpecimen> &hosts, const tgl_cell_list_config *cl
         // Wall reactions are kept when some axis has walls (on periodic
         // axes every reaction is zero).
         if (!grid.periodic[0] || !grid.periodic[1] || !grid.periodic[2]) {
-            if ((rc = w->alloc(&d.reaction, V))) return fail(rc);
+            if ((rc = w->alloc(&d.reaction, V)) || (rc = w->alloc(&d.reaction_next, V))) return fail(rc);
             if (cudaMemset(d.reaction, 0, V * sizeof(float4)) != cudaSuccess)
                 return fail(set_error(TGL_ERR_CUDA, "device initialisation failed"));
         }
@@ -922,7 +922,7 @@ int build_world(std::vector<HostSpecimen> &hosts, const tgl_cell_list_config *cl
     }
     w->lp.arena = arena;
     plan_launches(d, w->lp);
-    if (arena && !w->lp.fiber_lanes)
+    if (arena && (!w->lp.fiber_lanes || max_fiber > 256))
         return fail(set_error(TGL_ERR_UNSUPPORTED, "an arena needs fibers of at most 256 vertices"));
     *out = w;
     return 0;
