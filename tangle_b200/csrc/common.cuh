@@ -300,8 +300,12 @@ struct Control {
     // block to finish puts it back to 0.
     uint32_t next_batch;
     uint32_t cell_overflow;
-    // Contact lists: refresh pending, refreshes done.
+    // Contact lists: refresh pending (2: for new Verlet lists, not for a
+    // move), refreshes done; the skin the lists were made with and the listed
+    // passes they have served.
     uint32_t contact_state[2];
+    float contact_skin;
+    uint32_t contact_age;
     // Rebuild pipelines a batch graph's conditional node has run.
     uint32_t rebuild_bodies;
     // Steps a looped batch graph has begun (its WHILE node's counter).

@@ -104,10 +104,28 @@ __global__ void begin_batch_kernel(WorldDev w) {
     }
 }
 
-// Whether vertex v at (x, y, z) has moved more than half the contact skin
-// (less 0.1 %, a margin for rounding) from the contact lists' snapshot.
-__device__ inline bool contact_moved(const WorldDev &w, uint32_t v, float x, float y, float z) {
-    const float limit = 0.4995f * w.contact_skin;
+// The contact skin of the lists that a refresh makes. A narrow skin gives
+// short lists that every listed pass reads, a wide one (2.5 times it) fewer
+// refreshes, each of which walks the Verlet lists. With the motion of the
+// lists before, narrow lists would have lasted contact_skin / their skin
+// times as many passes. On the mid-size specimen a refresh takes 1.74 ms and
+// a listed pass 0.2 ms with 4 entries a segment or 0.33 ms with 7, so the two
+// cost the same where narrow lists last 7 passes: just below, lists of a
+// fresh packing live 2.3 passes; above, those of a relaxed one 20. Lists
+// that end with their Verlet lists say nothing about the motion. Contact
+// stage of 128 iterations from the initial packing with the narrow skin
+// alone 113.7 ms (57 refreshes), with this choice 90.8 ms; 64 iterations at
+// 2,000 fibers 10.4 -> 8.6 ms, 48 batched specimens 36.7 -> 32.8 ms; a
+// relaxed packing keeps the narrow skin (6.6 ms both).
+__device__ inline float next_contact_skin(const WorldDev &w, const Control *c) {
+    if (c->contact_state[0] == 2) return c->contact_skin == w.contact_wide ? w.contact_wide : w.contact_skin;
+    return w.contact_skin * (float)(c->contact_age + 1u) >= 7.0f * c->contact_skin ? w.contact_skin : w.contact_wide;
+}
+
+// Whether vertex v at (x, y, z) has moved more than half the contact lists'
+// skin (less 0.1 %, a margin for rounding) from their snapshot.
+__device__ inline bool contact_moved(const WorldDev &w, float skin, uint32_t v, float x, float y, float z) {
+    const float limit = 0.4995f * skin;
     const float4 c = w.contact_ref[v];
     const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
     return dx * dx + dy * dy + dz * dz > limit * limit;
@@ -126,7 +144,7 @@ __global__ void flag_displacement_kernel(WorldDev w) {
         float dx = p.x - r.x, dy = p.y - r.y, dz = p.z - r.z;
         far = dx * dx + dy * dy + dz * dz > md * md;
         if (A && far) flag_rebuild<A>(w, spec);
-        if (w.contact_skin > 0.0f && contact_moved(w, v, p.x, p.y, p.z)) {
+        if (w.contact_skin > 0.0f && contact_moved(w, ctl_of<A>(w, spec)->contact_skin, v, p.x, p.y, p.z)) {
             contact_far = true;
             if (A) flag_refresh<A>(w, spec);
         }
@@ -678,7 +696,7 @@ __device__ inline void finish_rebuild(Control *ctl) {
     if (ctl->neighbor_state[0] == 0) return;
     ctl->neighbor_state[0] = 0;
     ctl->neighbor_state[1] += 1;
-    ctl->contact_state[0] = 1;
+    ctl->contact_state[0] = 2;
 }
 
 template <bool A>
@@ -818,6 +836,14 @@ __device__ inline void assess_reduced_metrics(Control *c, const StepParams &sp, 
     c->acc[2] = 0;
 }
 
+// A refresh pass is over: the lists it made.
+__device__ inline void lists_made(const WorldDev &w, Control *c) {
+    c->contact_skin = next_contact_skin(w, c);
+    c->contact_age = 0;
+    c->contact_state[0] = 0;
+    c->contact_state[1] += 1;
+}
+
 // Contact pass modes: the Verlet lists as they are (CONTACT_FULL); the
 // Verlet lists plus a refresh of the contact lists and their snapshot
 // (CONTACT_REFRESH, run when the refresh flag is set); the contact lists
@@ -834,10 +860,10 @@ enum { CONTACT_FULL = 0, CONTACT_REFRESH = 1, CONTACT_LISTED = 2 };
 // block to finish runs assess_reduced_metrics (kernels.rs:129-162).
 //
 // Contact lists. A candidate can only produce a hit while its segments'
-// distance is below r1 + r2, and while no vertex has moved more than
-// contact_skin / 2 from a snapshot, no segment distance has shrunk by more
-// than contact_skin since it. So the Verlet-list entries whose distance at
-// the snapshot is within contact_skin of touching (within_contact_skin, a
+// distance is below r1 + r2, and while no vertex has moved more than half
+// the lists' contact skin from a snapshot, no segment distance has shrunk by
+// more than the skin since it. So the Verlet-list entries whose distance at
+// the snapshot is within the skin of touching (within_contact_skin, a
 // conservative test) hold every hit of every pass until a vertex moves
 // farther; the update kernel flags that, as it flags Verlet rebuilds, and a
 // Verlet rebuild forces a refresh. Hits are summed in ascending segment
@@ -859,6 +885,7 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
     __shared__ uint32_t kept_count[CONTACT_WARPS][32];
     __shared__ uint32_t hit_mask[CONTACT_WARPS][32];   // queue lanes holding each owner's hits; zero between rounds
     __shared__ uint32_t lane_spec[A ? CONTACT_WARPS : 1][32];
+    __shared__ float lane_skin[A && MODE == CONTACT_REFRESH ? CONTACT_WARPS : 1][32];  // of the owner's new lists
     __shared__ uint32_t warp_max[CONTACT_WARPS];
     __shared__ int is_last;
     if (gate && w.ctl->control[0] == 0) return;
@@ -871,7 +898,7 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t block = w.block;
     const uint32_t cblock = w.contact_block;
-    const float cskin = w.contact_skin;
+    const float cskin_world = !A && MODE == CONTACT_REFRESH ? next_contact_skin(w, w.ctl) : 0.0f;
     float4 *hg = home_geom[warp];
     uint32_t *pre = prefix[warp];
     float4 *qg = queue_geom[warp];
@@ -932,6 +959,8 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
         else if (valid && cstate == CONTACT_USE_VERLET) count = w.nbr_count[segment];
         const bool listed = MODE == CONTACT_LISTED ? valid && cstate != CONTACT_USE_SCAN : valid && count <= block;
         if (A) lane_spec[A ? warp : 0][lane] = my_spec;
+        if (A && MODE == CONTACT_REFRESH)
+            lane_skin[A && MODE == CONTACT_REFRESH ? warp : 0][lane] = next_contact_skin(w, ctl_of<A>(w, my_spec));
         uint32_t k = listed ? count : 0u;
         const uint32_t *source = w.nbr_list + (size_t)segment * block;
         if (MODE == CONTACT_LISTED) {
@@ -1018,6 +1047,7 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
                     const Grid &g = grid_of<A>(w, hspec);
                     const float line_eps = A ? w.specs[hspec].line_eps : line_eps_world;
                     if (MODE == CONTACT_REFRESH) {
+                        const float cskin = A ? lane_skin[A && MODE == CONTACT_REFRESH ? warp : 0][h] : cskin_world;
                         // Queue what may come within the contact skin; mark
                         // what passes the pass's own exact tests.
                         pass = contact_reach_wide(home, oa, ob, g, cskin, p2x, p2y, p2z, q2x, q2y, q2z, exact) &&
@@ -1054,7 +1084,8 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
                         hit = contact_solve(home, __float_as_uint(eb.w), ea.w, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z,
                                             sp.correction_fraction, sp.contact_aggregation, pt);
                     if (MODE == CONTACT_REFRESH)
-                        keep = within_contact_skin(home, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z, ea.w, cskin,
+                        keep = within_contact_skin(home, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z, ea.w,
+                                                   A ? lane_skin[A && MODE == CONTACT_REFRESH ? warp : 0][h] : cskin_world,
                                                    A ? w.specs[lane_spec[A ? warp : 0][h]].line_eps : line_eps_world);
                 }
                 if (MODE == CONTACT_REFRESH) {
@@ -1179,10 +1210,8 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
             Control *c = w.ctl;
             assess_reduced_metrics(c, sp, c->cell_overflow);
             c->done_blocks = 0;
-            if (MODE == CONTACT_REFRESH) {
-                c->contact_state[0] = 0;
-                c->contact_state[1] += 1;
-            }
+            if (MODE == CONTACT_REFRESH) lists_made(w, c);
+            if (MODE == CONTACT_LISTED) c->contact_age += 1;
             __threadfence();
         }
         return;
@@ -1196,10 +1225,10 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
     for (uint32_t p = threadIdx.x; p < w.P; p += blockDim.x) {
         Control *c = w.ctl + 1 + p;
         if (c->control[0] == 0) continue;
-        if (MODE == CONTACT_REFRESH && c->contact_state[0]) {  // refreshed in this pass
-            c->contact_state[0] = 0;
-            c->contact_state[1] += 1;
-        }
+        if (MODE == CONTACT_REFRESH && c->contact_state[0])  // refreshed in this pass
+            lists_made(w, c);
+        else
+            c->contact_age += 1;
         assess_reduced_metrics(c, sp, w.ctl->cell_overflow);
         if (c->control[0]) any_active = 1;
     }
@@ -1339,6 +1368,7 @@ __global__ void __launch_bounds__(256) fiber_kernel(WorldDev w, StepParams sp) {
     float4 *St = T + maxv;                             // static vertex data
     const Grid &g = w.grid;
     const float md = 0.5f * w.skin;
+    const float contact_skin = w.ctl->contact_skin;
     uint32_t smax = 0, cmax = 0;
     bool far = false;
     bool contact_far = false;
@@ -1525,7 +1555,7 @@ __global__ void __launch_bounds__(256) fiber_kernel(WorldDev w, StepParams sp) {
             float4 r = w.ref_pos[v0 + i];
             float dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z;
             if (dx * dx + dy * dy + dz * dz > md * md) far = true;
-            if (contact_lists && contact_moved(w, v0 + i, x.x, x.y, x.z)) contact_far = true;
+            if (contact_lists && contact_moved(w, contact_skin, v0 + i, x.x, x.y, x.z)) contact_far = true;
             if (i > 0 && i + 1 < n) {
                 float maximum = St[i].x;
                 if (maximum > 0.0f) {
@@ -2291,6 +2321,7 @@ __global__ void __launch_bounds__(128, A ? 6 : 4) fiber_lanes_kernel(WorldDev w,
             if (f == TGL_NONE) continue;
             const uint32_t fspec = spec_of_fiber<A>(w, f);
             const float md = 0.5f * skin_of<A>(w, fspec);
+            const float contact_skin = ctl_of<A>(w, fspec)->contact_skin;
             const uint2 span = w.fiber_vspan[f];
             const uint32_t v0 = span.x;
             const int n = (int)span.y;
@@ -2304,7 +2335,7 @@ __global__ void __launch_bounds__(128, A ? 6 : 4) fiber_lanes_kernel(WorldDev w,
                 const float4 r = w.ref_pos[v0 + i];
                 const float dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z;
                 if (dx * dx + dy * dy + dz * dz > md * md) far = true;
-                if (contact_lists && contact_moved(w, v0 + i, x.x, x.y, x.z)) contact_far = true;
+                if (contact_lists && contact_moved(w, contact_skin, v0 + i, x.x, x.y, x.z)) contact_far = true;
                 if (i > 0 && i + 1 < n) {
                     const float maximum = lanes_limit(x);
                     if (maximum > 0.0f) {
@@ -2450,6 +2481,7 @@ __global__ void __launch_bounds__(256) rigid_kernel(WorldDev w, StepParams sp) {
         if (!A) formation_targets_staged(w, f, w.pos + v0, (int)n, v0, lane);
         smax = max(smax, __float_as_uint(fmaxf(applied, 0.0f)));
         const float md = 0.5f * skin_of<A>(w, spec);
+        const float contact_skin = ctl_of<A>(w, spec)->contact_skin;
         const float radius = w.seg_static[s0].x;
         const float4 *P = w.pos + v0;
         for (uint32_t i = lane; i < n; i += 32) {
@@ -2457,7 +2489,7 @@ __global__ void __launch_bounds__(256) rigid_kernel(WorldDev w, StepParams sp) {
             const float4 r = w.ref_pos[v0 + i];
             const float dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z;
             if (dx * dx + dy * dy + dz * dz > md * md) far = true;
-            if (contact_lists && contact_moved(w, v0 + i, x.x, x.y, x.z)) contact_far = true;
+            if (contact_lists && contact_moved(w, contact_skin, v0 + i, x.x, x.y, x.z)) contact_far = true;
             if (i > 0 && i + 1 < n) {
                 const float maximum = w.vtx_static[v0 + i].x;
                 if (maximum > 0.0f) {

@@ -36,11 +36,12 @@ struct WorldDev {
     uint32_t max_fiber;  // most vertices in one fiber
     float skin;          // neighbor skin
     // Contact lists: per cell-list slot, the Verlet-list entries that lie
-    // within contact_skin of touching at the contact_ref snapshot (0 = off).
-    float contact_skin;
+    // within a contact skin of touching at the contact_ref snapshot: this one
+    // (0 = off) or contact_wide (next_contact_skin chooses).
+    float contact_skin, contact_wide;
     uint32_t contact_block;  // entries per slot
-    // Longest half length for which a pair within reach + contact_skin has
-    // one minimum image (L/2 > 2 H + 2 r_max + contact_skin on every periodic
+    // Longest half length for which a pair within reach + contact_wide has
+    // one minimum image (L/2 > 2 H + 2 r_max + contact_wide on every periodic
     // axis); a longer segment makes every pass refresh (read the Verlet list).
     float contact_half_limit;
     Grid grid;

@@ -905,7 +905,8 @@ int build_world(std::vector<HostSpecimen> &hosts, const tgl_cell_list_config *cl
     ctl.metrics[1] = 0.0f;
     ctl.metrics[2] = INFINITY;
     ctl.neighbor_state[0] = 1;  // lists start stale (world.rs:516-517)
-    ctl.contact_state[0] = 1;
+    ctl.contact_state[0] = 2;
+    ctl.contact_skin = d.contact_skin;
     std::vector<Control> controls(arena ? count + 1 : 1, ctl);
     if (cudaMemcpy(d.ctl, controls.data(), controls.size() * sizeof(Control), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(d.corr, 0, 2 * (size_t)S * sizeof(float4)) != cudaSuccess ||
@@ -1697,7 +1698,7 @@ int tgl_world_compact_cell(tgl_world *w, const float new_lower[3], const float n
             if (d.grid.periodic[a])
                 d.contact_half_limit =
                     std::fmin(d.contact_half_limit,
-                              0.999f * 0.5f * (0.5f * d.grid.length[a] - 2.0f * w->maximum_radius - d.contact_skin));
+                              0.999f * 0.5f * (0.5f * d.grid.length[a] - 2.0f * w->maximum_radius - d.contact_wide));
     }
     plan_launches(d, w->lp);
     w->launches += launch_refresh_geometry(d, w->stream);
@@ -1805,13 +1806,18 @@ void set_contact_skin(tgl_world *w, float fraction) {
     // than the contact skin: with every half length below H, pairs within
     // reach + contact skin are closer than half a box length on every
     // periodic axis, so H = (L/2 - 2 r_max - contact_skin) / 2, less 0.1 %,
-    // over every specimen's box.
-    d.contact_half_limit = INFINITY;
-    for (const Grid &g : w->contact_grids)
-        for (int a = 0; a < 3; ++a)
-            if (g.periodic[a])
-                d.contact_half_limit = std::fmin(
-                    d.contact_half_limit, 0.999f * 0.5f * (0.5f * g.length[a] - 2.0f * w->maximum_radius - d.contact_skin));
+    // over every specimen's box. The wide skin where it leaves room.
+    d.contact_wide = std::fmin(2.5f * d.contact_skin, std::fmax(w->contact_skin_base, d.contact_skin));
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        d.contact_half_limit = INFINITY;
+        for (const Grid &g : w->contact_grids)
+            for (int a = 0; a < 3; ++a)
+                if (g.periodic[a])
+                    d.contact_half_limit = std::fmin(
+                        d.contact_half_limit, 0.999f * 0.5f * (0.5f * g.length[a] - 2.0f * w->maximum_radius - d.contact_wide));
+        if (d.contact_half_limit > 0.5f * w->maximum_length) break;
+        d.contact_wide = d.contact_skin;
+    }
     if (!(d.contact_half_limit > 0.5f * w->maximum_length)) d.contact_skin = 0.0f;  // no room: full lists every pass
     w->contact_fraction = d.contact_skin > 0.0f ? fraction : 0.0f;
 }
