@@ -1,8 +1,8 @@
-// umma_gemm_tma.cuh -- persistent BF16 products for K-major operands:
+// umma_gemm_tma.cuh -- persistent BF16 products for a K-major A:
 // TMA-fed, pipelined, two tensor-memory accumulators.
 //
-// D[M x N] = A[M x K] B[N x K]^T (+ the epilogue of umma_gemm.cuh), both
-// operands K-major (a[m * lda + k], b[n * ldb + k]), N % 16 == 0, N <= 256,
+// D[M x N] = A[M x K] B[N x K]^T (+ the epilogue of umma_gemm.cuh), the
+// operands K-major (a[m * lda + k], b[n * ldb + k]; B see below), N % 16 == 0, N <= 256,
 // K % 8 == 0. Each CTA walks the 128-row tiles blockIdx.x, + gridDim.x, ...
 // with three roles:
 //   warp 0 (one lane): the producer. For each 64-wide contraction chunk it
@@ -31,6 +31,11 @@
 //     residual are applied and the results stored as 64-byte row pieces
 //     (f32) or 32-byte ones (bf16) instead of one 16-byte piece per row and
 //     lane. Then it arrives on the accumulator's "empty" mbarrier.
+// An MN-major B (b[k * ldb + n], the weights of a data gradient) cannot come
+// through those boxes: RESIDENT_B keeps all of it in shared memory, written
+// once per CTA in the same swizzled layout, and the stages hold A alone: 4 M x
+// 64 -> 80 in f32 0.38 ms, -> 64 in f32 and bf16 with a mask 0.87 ms, against
+// 0.78 and 1.86 ms on the staged kernel.
 // Every mbarrier wait is bounded: one that gives up records an error and
 // the CTA stops issuing work; before it exits, the producer waits (bounded)
 // for its loads still in flight and the MMA issuer for its last commit, and
@@ -60,10 +65,16 @@ __host__ __device__ inline uint32_t tma_stage_bytes(int n) {
 constexpr int TMA_EPI_STRIDE = 20;
 constexpr uint32_t TMA_EPI_BYTES = 4u * 32u * TMA_EPI_STRIDE * 4u;
 
-// Dynamic shared memory of the kernel: the stages, the epilogue slices and
-// the slack that lets the first stage start on a 1024-byte boundary.
+// Dynamic shared memory of the kernel: the stages, a resident B's chunks, the
+// epilogue slices and the slack that lets the first stage start on a
+// 1024-byte boundary.
 __host__ __device__ inline uint32_t tma_smem_bytes(int n) {
     return (uint32_t)TMA_GEMM_STAGES * tma_stage_bytes(n) + TMA_EPI_BYTES + 1024u;
+}
+__host__ __device__ inline uint32_t tma_resident_smem_bytes(int n, int64_t k) {
+    const uint32_t chunks = (uint32_t)((k + GEMM_KC - 1) / GEMM_KC);
+    return (uint32_t)TMA_GEMM_STAGES * tma_stage_bytes(0) + chunks * (tma_stage_bytes(n) - tma_stage_bytes(0)) +
+           TMA_EPI_BYTES + 1024u;
 }
 
 // tcgen05 shared-memory descriptor of a K-major operand in the 128-byte
@@ -103,6 +114,7 @@ __device__ inline void tma_load_2d(uint32_t dst, const CUtensorMap *map, int32_t
         : "memory");
 }
 
+template <bool RESIDENT_B>
 __global__ void __launch_bounds__(TMA_GEMM_THREADS, 1)
     umma_gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          GemmArgs g) {
@@ -113,7 +125,8 @@ __global__ void __launch_bounds__(TMA_GEMM_THREADS, 1)
     __shared__ volatile int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = g.n;
-    const uint32_t stage_bytes = tma_stage_bytes(n);
+    const uint32_t stage_bytes = tma_stage_bytes(RESIDENT_B ? 0 : n);
+    const uint32_t b_bytes = tma_stage_bytes(n) - tma_stage_bytes(0);  // one chunk of B
     const uint32_t smem0 = (smem_u32(tma_smem) + 1023u) & ~1023u;
     const int64_t tiles = ((int64_t)g.m + GEMM_BM - 1) / GEMM_BM;
     const int64_t chunks = (g.k + GEMM_KC - 1) / GEMM_KC;
@@ -136,6 +149,23 @@ __global__ void __launch_bounds__(TMA_GEMM_THREADS, 1)
         asm volatile("fence.mbarrier_init.release.cluster;");
         failed = 0;
     }
+    uint8_t *const resident = tma_smem + (smem0 - smem_u32(tma_smem)) + TMA_GEMM_STAGES * stage_bytes;
+    if (RESIDENT_B) {
+        // Contraction row c holds element c % 64 of chunk c / 64 for every
+        // operand row r (a row past K is zero).
+        for (int64_t v = threadIdx.x; v < chunks * GEMM_KC * (n / 8); v += blockDim.x) {
+            const int64_t c = v / (n / 8);
+            const int r0 = (int)(v % (n / 8)) * 8, cc = (int)(c % GEMM_KC);
+            uint4 val = make_uint4(0u, 0u, 0u, 0u);
+            if (c < g.k) val = *reinterpret_cast<const uint4 *>(g.b + c * g.ldb + r0);
+            const uint16_t *element = reinterpret_cast<const uint16_t *>(&val);
+            uint8_t *chunk = resident + (c / GEMM_KC) * b_bytes;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)  // r0 % 8 is 0: row j of an 8-row atom
+                *reinterpret_cast<uint16_t *>(chunk + (r0 + j) * 128 + (((cc >> 3) ^ j) << 4) + (cc & 7) * 2) = element[j];
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -156,11 +186,11 @@ __global__ void __launch_bounds__(TMA_GEMM_THREADS, 1)
                     // with zeros and counts toward the stage's bytes.
                     const int32_t x = (int32_t)(c * GEMM_KC);
                     const uint32_t full = smem_u32(&full_bar[stage]);
-                    mbar_expect_tx(full, (uint32_t)(GEMM_KC * 2) * (uint32_t)(GEMM_BM + n));
+                    mbar_expect_tx(full, (uint32_t)(GEMM_KC * 2) * (uint32_t)(RESIDENT_B ? GEMM_BM : GEMM_BM + n));
                     const uint32_t sa = smem0 + stage * stage_bytes;
                     const uint32_t sb = sa + GEMM_BM * GEMM_KC * 2;
                     tma_load_2d(sa, &map_a, x, (int32_t)(t * GEMM_BM), full);
-                    tma_load_2d(sb, &map_b, x, 0, full);
+                    if (!RESIDENT_B) tma_load_2d(sb, &map_b, x, 0, full);
                     ++issued[stage];
                     if (++stage == TMA_GEMM_STAGES) {
                         stage = 0;
@@ -201,7 +231,8 @@ __global__ void __launch_bounds__(TMA_GEMM_THREADS, 1)
                     const int kk = (int)(g.k - k0 < GEMM_KC ? g.k - k0 : GEMM_KC);
                     const int steps = (kk + 15) / 16;
                     const uint32_t sa = smem0 + stage * stage_bytes;
-                    const uint32_t sb = sa + GEMM_BM * GEMM_KC * 2;
+                    const uint32_t sb = RESIDENT_B ? smem0 + TMA_GEMM_STAGES * stage_bytes + (uint32_t)c * b_bytes
+                                                   : sa + GEMM_BM * GEMM_KC * 2;
                     for (int s = 0; s < steps; ++s) {
                         const uint64_t da = smem_desc_sw128(sa + 32u * (uint32_t)s);
                         const uint64_t db = smem_desc_sw128(sb + 32u * (uint32_t)s);
@@ -237,8 +268,7 @@ __global__ void __launch_bounds__(TMA_GEMM_THREADS, 1)
     } else {
         // Epilogue: warps 2-5; this warp's tensor-memory lanes and tile rows.
         const int quarter = warp & 3;
-        float *slice = reinterpret_cast<float *>(tma_smem + (smem0 - smem_u32(tma_smem)) +
-                                                 TMA_GEMM_STAGES * stage_bytes) +
+        float *slice = reinterpret_cast<float *>(resident + (RESIDENT_B ? (uint32_t)chunks * b_bytes : 0u)) +
                        quarter * 32 * TMA_EPI_STRIDE;
         const int cq = 4 * (lane & 3);  // this lane's 4 columns of a slice
         uint32_t acc = 0, acc_phase[2] = {0u, 0u};

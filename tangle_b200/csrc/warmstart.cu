@@ -61,25 +61,31 @@ bool kmajor_map(CUtensorMap *map, const void *base, int64_t rows, int64_t k, int
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The persistent TMA kernel for products whose operands are both K-major and
-// whose contraction is not split; 0 when it ran, 1 when this product or the
-// driver calls for the staged kernel instead, or an error code.
+// The persistent TMA kernel for products with a K-major A and an unsplit
+// contraction (an MN-major B as long as it fits in shared memory beside the
+// stages); 0 when it ran, 1 when this product or the driver calls for the
+// staged kernel instead, or an error code.
 int gemm_tma(const tgl_gemm *p, const tgl::GemmArgs &g, cudaStream_t stream) {
-    if (p->a_mn || p->b_mn || p->k_split > 0 || p->k <= 0 || std::getenv("TGL_GEMM_STAGED")) return 1;
+    if (p->a_mn || p->k_split > 0 || p->k <= 0 || std::getenv("TGL_GEMM_STAGED")) return 1;
     if (p->m > 0x7FFFFF80 || p->k > 0x7FFFFFF0) return 1;  // TMA coordinates are 32-bit
+    if (p->b_mn && p->k > 512) return 1;
+    const size_t smem = p->b_mn ? tgl::tma_resident_smem_bytes(p->n, p->k) : tgl::tma_smem_bytes(p->n);
+    if (smem > 220u * 1024u) return 1;
     CUtensorMap map_a, map_b;
-    if (!kmajor_map(&map_a, p->a, p->m, p->k, p->lda, tgl::GEMM_BM) ||
-        !kmajor_map(&map_b, p->b, p->n, p->k, p->ldb, p->n))
+    if (!kmajor_map(&map_a, p->a, p->m, p->k, p->lda, tgl::GEMM_BM)) return 1;
+    if (p->b_mn)
+        map_b = map_a;  // not read
+    else if (!kmajor_map(&map_b, p->b, p->n, p->k, p->ldb, p->n))
         return 1;
-    const size_t smem = tgl::tma_smem_bytes(p->n);
     static std::once_flag once;
     static int sms = 0;
     std::call_once(once, [] {
         int device = 0;
         cudaGetDevice(&device);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaFuncSetAttribute(tgl::umma_gemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(tgl::umma_gemm_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)tgl::tma_smem_bytes(256));
+        cudaFuncSetAttribute(tgl::umma_gemm_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     });
     int cols = 32;
     while (cols < p->n) cols <<= 1;
@@ -87,7 +93,10 @@ int gemm_tma(const tgl_gemm *p, const tgl::GemmArgs &g, cudaStream_t stream) {
     const int per_sm = std::max(1, std::min(by_smem, by_tmem));
     const int64_t tiles = ((int64_t)p->m + tgl::GEMM_BM - 1) / tgl::GEMM_BM;
     const int blocks = (int)std::min<int64_t>(tiles, (int64_t)std::max(sms, 1) * per_sm);
-    tgl::umma_gemm_tma_kernel<<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
+    if (p->b_mn)
+        tgl::umma_gemm_tma_kernel<true><<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
+    else
+        tgl::umma_gemm_tma_kernel<false><<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return gemm_error(TGL_ERR_CUDA, std::string("tgl_gemm_bf16: ") + cudaGetErrorString(e));
     return 0;
@@ -147,13 +156,12 @@ extern "C" int tgl_gemm_bf16(const tgl_gemm *p, void *stream) {
         const int rc = gemm_tma(p, g, static_cast<cudaStream_t>(stream));
         if (rc != 1) return rc;
     }
-    const size_t smem = (size_t)tgl::GEMM_BM * tgl::GEMM_KC * 2 + (size_t)p->n * tgl::GEMM_KC * 2;
-    static bool configured = false;
-    if (!configured) {
+    const size_t smem = (size_t)tgl::GEMM_STAGES * (tgl::GEMM_BM + p->n) * tgl::GEMM_KC * 2;
+    static std::once_flag configured;
+    std::call_once(configured, [] {
         cudaFuncSetAttribute(tgl::umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)((size_t)tgl::GEMM_BM * tgl::GEMM_KC * 2 + 256 * tgl::GEMM_KC * 2));
-        configured = true;
-    }
+                             tgl::GEMM_STAGES * (tgl::GEMM_BM + 256) * tgl::GEMM_KC * 2);
+    });
     dim3 grid((unsigned)((p->m + tgl::GEMM_BM - 1) / tgl::GEMM_BM), (unsigned)splits);
     tgl::umma_gemm_kernel<<<grid, tgl::GEMM_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(g);
     cudaError_t e = cudaGetLastError();
@@ -352,26 +360,68 @@ __global__ void graph_fill_kernel(WorldDev w, GraphBuffers g, float cutoff) {
     }
 }
 
-// Sort each segment's incoming edges (sources below it) by source, carrying
-// every per-edge record; the twins of moved edges are fixed afterwards.
+// One edge's records, as the sort moves them.
+struct EdgeRecord {
+    int32_t src, twin;
+    float s, t, depth;
+    uint4 f0, f1;
+};
+
+__device__ inline EdgeRecord read_edge(const GraphBuffers &g, int64_t e) {
+    const uint4 *f = reinterpret_cast<const uint4 *>(g.edge_features + e * MP_EDGE_FEATURES);
+    return {g.src[e], g.twin[e], g.s[e], g.t[e], g.depth[e], f[0], f[1]};
+}
+
+__device__ inline void write_record(const GraphBuffers &g, int64_t e, const EdgeRecord &r) {
+    g.src[e] = r.src;
+    g.twin[e] = r.twin;
+    g.s[e] = r.s;
+    g.t[e] = r.t;
+    g.depth[e] = r.depth;
+    uint4 *f = reinterpret_cast<uint4 *>(g.edge_features + e * MP_EDGE_FEATURES);
+    f[0] = r.f0;
+    f[1] = r.f1;
+}
+
+// Sort each segment's incoming edges (sources below it, each once) by source,
+// carrying every per-edge record; the twins of moved edges are fixed
+// afterwards. One warp per segment: up to 64 edges (20 on average) are read
+// into registers, two a lane, ranked by counting smaller sources and written
+// to their ranks; more are insertion-sorted by one lane. 0.73 ms for 4.1 M
+// incoming edges; one thread per segment swapping neighbors in global memory
+// took 6.1 ms (bound by the latency of its serial swaps).
 __global__ void graph_sort_kernel(WorldDev w, GraphBuffers g) {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.S; b += gridDim.x * blockDim.x) {
-        const int64_t lo = g.offsets[b], n = g.in_count[b];
-        for (int64_t i = 1; i < n; ++i) {
-            for (int64_t j = i; j > 0 && g.src[lo + j] < g.src[lo + j - 1]; --j) {
-                const int64_t x = lo + j, y = lo + j - 1;
-                int32_t ti = g.src[x]; g.src[x] = g.src[y]; g.src[y] = ti;
-                ti = g.twin[x]; g.twin[x] = g.twin[y]; g.twin[y] = ti;
-                float tf = g.s[x]; g.s[x] = g.s[y]; g.s[y] = tf;
-                tf = g.t[x]; g.t[x] = g.t[y]; g.t[y] = tf;
-                tf = g.depth[x]; g.depth[x] = g.depth[y]; g.depth[y] = tf;
-                uint4 *fx = reinterpret_cast<uint4 *>(g.edge_features + x * MP_EDGE_FEATURES);
-                uint4 *fy = reinterpret_cast<uint4 *>(g.edge_features + y * MP_EDGE_FEATURES);
-                const uint4 a0 = fx[0], a1 = fx[1];
-                fx[0] = fy[0];
-                fx[1] = fy[1];
-                fy[0] = a0;
-                fy[1] = a1;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < w.S; b += warps) {
+        const int64_t lo = g.offsets[b];
+        const int n = (int)g.in_count[b];
+        if (n < 2) continue;
+        if (n <= 64) {
+            EdgeRecord r0, r1;
+            r0.src = r1.src = 0x7FFFFFFF;
+            if (lane < n) r0 = read_edge(g, lo + lane);
+            if (32 + lane < n) r1 = read_edge(g, lo + 32 + lane);
+            int rank0 = 0, rank1 = 0;
+            for (int j = 0; j < min(n, 32); ++j) {
+                const int32_t other = __shfl_sync(WFULL, r0.src, j);
+                rank0 += other < r0.src;
+                rank1 += other < r1.src;
+            }
+            for (int j = 32; j < n; ++j) {
+                const int32_t other = __shfl_sync(WFULL, r1.src, j - 32);
+                rank0 += other < r0.src;
+                rank1 += other < r1.src;
+            }
+            __syncwarp();
+            if (lane < n) write_record(g, lo + rank0, r0);
+            if (32 + lane < n) write_record(g, lo + rank1, r1);
+        } else if (lane == 0) {
+            for (int i = 1; i < n; ++i) {
+                const EdgeRecord r = read_edge(g, lo + i);
+                int j = i;
+                for (; j > 0 && g.src[lo + j - 1] > r.src; --j) write_record(g, lo + j, read_edge(g, lo + j - 1));
+                write_record(g, lo + j, r);
             }
         }
     }
@@ -548,7 +598,7 @@ int launch_graph_offsets(const WorldDev &w, const GraphBuffers &g, cudaStream_t 
 
 void launch_graph_fill(const WorldDev &w, const GraphBuffers &g, float cutoff, cudaStream_t st) {
     graph_fill_kernel<<<blocks_for(w.S, 8, 148 * 32), 256, 0, st>>>(w, g, cutoff);
-    graph_sort_kernel<<<blocks_for(w.S, 256, 1 << 20), 256, 0, st>>>(w, g);
+    graph_sort_kernel<<<blocks_for(w.S, 8, 148 * 32), 256, 0, st>>>(w, g);
     graph_twin_kernel<<<148 * 8, 256, 0, st>>>(w, g);
 }
 
@@ -585,17 +635,30 @@ namespace {
 
 constexpr int MP_ROWS_PER_CHUNK = 4096;  // rows per partial in column sums
 
-// One warp per edge: lanes cover the 64 embedding columns two at a time.
-__global__ void edge_inputs_kernel(MpGraph g, const float *h, __nv_bfloat16 *x, int64_t ld) {
+// Lanes cover the 64 embedding columns two at a time. A warp takes 32 edges:
+// their sources and parameters in one read, then edge after edge, so that
+// only the embedding rows are waited for (one edge per warp and step waited
+// for its source, its vertex and its rows in turn: 0.87 ms for 8.1 M edges).
+__global__ void edge_inputs_kernel(MpGraph g, const float *__restrict__ h, __nv_bfloat16 *__restrict__ x, int64_t ld) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t e = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); e < g.E; e += warps) {
-        const int32_t v0 = g.seg_v0[g.src[e]];
-        const float t = g.t[e];
-        const float2 a = reinterpret_cast<const float2 *>(h + (int64_t)v0 * MP_HIDDEN)[lane];
-        const float2 b = reinterpret_cast<const float2 *>(h + (int64_t)(v0 + 1) * MP_HIDDEN)[lane];
-        reinterpret_cast<__nv_bfloat162 *>(x + e * ld)[lane] =
-            __floats2bfloat162_rn((1.0f - t) * a.x + t * b.x, (1.0f - t) * a.y + t * b.y);
+    for (int64_t e0 = 32 * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)); e0 < g.E; e0 += 32 * warps) {
+        int32_t my_v0 = 0;
+        float my_t = 0.0f;
+        if (e0 + lane < g.E) {
+            my_v0 = g.seg_v0[g.src[e0 + lane]];
+            my_t = g.t[e0 + lane];
+        }
+        const int count = (int)(g.E - e0 < 32 ? g.E - e0 : 32);
+#pragma unroll 4
+        for (int j = 0; j < count; ++j) {
+            const int32_t v0 = __shfl_sync(WFULL, my_v0, j);
+            const float t = __shfl_sync(WFULL, my_t, j);
+            const float2 a = reinterpret_cast<const float2 *>(h + (int64_t)v0 * MP_HIDDEN)[lane];
+            const float2 b = reinterpret_cast<const float2 *>(h + (int64_t)(v0 + 1) * MP_HIDDEN)[lane];
+            reinterpret_cast<__nv_bfloat162 *>(x + (e0 + j) * ld)[lane] =
+                __floats2bfloat162_rn((1.0f - t) * a.x + t * b.x, (1.0f - t) * a.y + t * b.y);
+        }
     }
 }
 
@@ -610,30 +673,77 @@ __device__ inline float vertex_weight(const MpGraph &g, int4 l) {
     return w;
 }
 
-// One warp per vertex: [h, the weighted mean of the messages into its two
-// segments (weights: its share, s or 1 - s), mean of the fiber neighbors' h].
-__global__ void node_inputs_kernel(MpGraph g, const float *h, const float *m, __nv_bfloat16 *x) {
+// Sums over the edges into segment c, in order, for its two vertices: `near`
+// takes the first vertex's share (1 - p) of each row, `far` the second's (p).
+struct SegmentSums {
+    float2 sum;
+    float weight;
+};
+
+template <typename Row, typename Share>
+__device__ inline void add_segment(const MpGraph &g, int32_t c, Row row, Share share, SegmentSums &near, SegmentSums &far) {
+    const int32_t end = g.offsets[c + 1];
+#pragma unroll 4
+    for (int32_t e = g.offsets[c]; e < end; ++e) {
+        const float p = share(e), q = 1.0f - p;
+        const float2 r = row(e);
+        near.sum.x += q * r.x;
+        near.sum.y += q * r.y;
+        near.weight += q;
+        far.sum.x += p * r.x;
+        far.sum.y += p * r.y;
+        far.weight += p;
+    }
+}
+
+constexpr int MP_RUN = 8;  // consecutive vertices of one warp's walk
+
+// A warp's walk over MP_RUN consecutive vertices: visit(v, links, sums) with
+// each vertex's sums over the edges into its two segments, the one before it
+// first. Consecutive vertices of a fiber share a segment, whose edges are
+// then read once for both (in the order of the sums: a vertex's second
+// segment adds to what its first gave).
+template <typename Row, typename Share, typename Visit>
+__device__ inline void walk_vertices(const MpGraph &g, int64_t first, Row row, Share share, Visit visit) {
+    const SegmentSums zero = {make_float2(0.0f, 0.0f), 0.0f};
+    SegmentSums carried = zero;
+    int32_t carried_segment = -1;
+    const int64_t end = first + MP_RUN < g.V ? first + MP_RUN : g.V;
+    for (int64_t v = first; v < end; ++v) {
+        const int4 l = g.links[v];
+        SegmentSums sums = zero;
+        if (l.z >= 0) {
+            if (l.z != carried_segment) {
+                carried = zero;
+                SegmentSums unused = zero;
+                add_segment(g, l.z, row, share, unused, carried);
+            }
+            sums = carried;
+        }
+        carried = zero;
+        carried_segment = l.w;
+        if (l.w >= 0) add_segment(g, l.w, row, share, sums, carried);
+        visit(v, l, sums);
+    }
+}
+
+// Per vertex: [h, the weighted mean of the messages into its two segments
+// (weights: its share, s or 1 - s), mean of the fiber neighbors' h]. Bound by
+// the messages' bytes (256 a row): 0.76 ms for 8.1 M edges (2.7 TB/s); a warp
+// per vertex, which read each message for both vertices of its segment and
+// the weights twice, took 1.02 ms. (The same walk over the edges out of a
+// vertex, whose rows lie anywhere, was slower than a warp per vertex: 0.58
+// against 0.51 ms in edge_inputs_backward_kernel.)
+__global__ void node_inputs_kernel(MpGraph g, const float *__restrict__ h, const float *__restrict__ m,
+                                   __nv_bfloat16 *__restrict__ x) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t v = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); v < g.V; v += warps) {
-        const int4 l = g.links[v];
+    const auto row_of = [&](int32_t e) { return reinterpret_cast<const float2 *>(m + (int64_t)e * MP_HIDDEN)[lane]; };
+    const auto share_of = [&](int32_t e) { return g.s[e]; };
+    const auto visit = [&](int64_t v, int4 l, const SegmentSums &sums) {
         const float2 hv = reinterpret_cast<const float2 *>(h + v * MP_HIDDEN)[lane];
-        float2 agg = make_float2(0.0f, 0.0f);
-        if (l.z >= 0)
-            for (int32_t e = g.offsets[l.z]; e < g.offsets[l.z + 1]; ++e) {
-                const float w = g.s[e];
-                const float2 me = reinterpret_cast<const float2 *>(m + (int64_t)e * MP_HIDDEN)[lane];
-                agg.x += w * me.x;
-                agg.y += w * me.y;
-            }
-        if (l.w >= 0)
-            for (int32_t e = g.offsets[l.w]; e < g.offsets[l.w + 1]; ++e) {
-                const float w = 1.0f - g.s[e];
-                const float2 me = reinterpret_cast<const float2 *>(m + (int64_t)e * MP_HIDDEN)[lane];
-                agg.x += w * me.x;
-                agg.y += w * me.y;
-            }
-        const float norm = 1.0f / fmaxf(vertex_weight(g, l), 1.0f);
+        float2 agg = sums.sum;
+        const float norm = 1.0f / fmaxf(sums.weight, 1.0f);
         agg.x *= norm;
         agg.y *= norm;
         float2 nb = make_float2(0.0f, 0.0f);
@@ -656,7 +766,9 @@ __global__ void node_inputs_kernel(MpGraph g, const float *h, const float *m, __
         row[lane] = __floats2bfloat162_rn(hv.x, hv.y);
         row[32 + lane] = __floats2bfloat162_rn(agg.x, agg.y);
         row[64 + lane] = __floats2bfloat162_rn(nb.x, nb.y);
-    }
+    };
+    for (int64_t run = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); run * MP_RUN < g.V; run += warps)
+        walk_vertices(g, run * MP_RUN, row_of, share_of, visit);
 }
 
 // dH[v] += dX[v, 0:64] + sum over fiber neighbors u of dX[u, 128:192] / count(u);
@@ -680,16 +792,26 @@ __global__ void node_inputs_backward_kernel(MpGraph g, const float *dx, float *d
         const float2 old = *out;
         *out = make_float2(old.x + acc.x, old.y + acc.y);
     }
-    for (int64_t e = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); e < g.E; e += warps) {
-        const int32_t v0 = g.seg_v0[g.dst[e]];
-        const float s = g.s[e];
-        const float wa = (1.0f - s) / fmaxf(vertex_weight(g, g.links[v0]), 1.0f);
-        const float wb = s / fmaxf(vertex_weight(g, g.links[v0 + 1]), 1.0f);
+    // The edges into a segment share its two vertices' rows and weights: 0.38
+    // ms for 4 M edges (an edge at a time, each with both weights summed anew,
+    // 3.9 ms).
+    for (int64_t c = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); c < g.S; c += warps) {
+        const int32_t begin = g.offsets[c], end = g.offsets[c + 1];
+        if (begin == end) continue;
+        const int32_t v0 = g.seg_v0[c];
+        const float na = fmaxf(vertex_weight(g, g.links[v0]), 1.0f);
+        const float nb = fmaxf(vertex_weight(g, g.links[v0 + 1]), 1.0f);
         const float2 a = reinterpret_cast<const float2 *>(dx + (int64_t)v0 * 3 * MP_HIDDEN + MP_HIDDEN)[lane];
         const float2 b = reinterpret_cast<const float2 *>(dx + (int64_t)(v0 + 1) * 3 * MP_HIDDEN + MP_HIDDEN)[lane];
-        const float2 d = make_float2(wa * a.x + wb * b.x, wa * a.y + wb * b.y);
-        reinterpret_cast<__nv_bfloat162 *>(dm + e * MP_HIDDEN)[lane] = __floats2bfloat162_rn(d.x, d.y);
-        if (dm32) reinterpret_cast<float2 *>(dm32 + e * MP_HIDDEN)[lane] = d;
+#pragma unroll 4
+        for (int64_t e = begin; e < end; ++e) {
+            const float s = g.s[e];
+            const float wa = (1.0f - s) / na;
+            const float wb = s / nb;
+            const float2 d = make_float2(wa * a.x + wb * b.x, wa * a.y + wb * b.y);
+            reinterpret_cast<__nv_bfloat162 *>(dm + e * MP_HIDDEN)[lane] = __floats2bfloat162_rn(d.x, d.y);
+            if (dm32) reinterpret_cast<float2 *>(dm32 + e * MP_HIDDEN)[lane] = d;
+        }
     }
 }
 
@@ -731,12 +853,16 @@ __global__ void edge_inputs_backward_kernel(MpGraph g, const float *dx, int64_t 
 
 // Column sums in two passes: partial[chunk][j] over MP_ROWS_PER_CHUNK rows,
 // then the chunks in order.
-__global__ void column_partials_kernel(const float *x, int64_t rows, int32_t n, int64_t ld, float *partial) {
+__global__ void column_partials_kernel(const float *__restrict__ x, int64_t rows, int32_t n, int64_t ld,
+                                       float *__restrict__ partial) {
     const int64_t chunk = blockIdx.y;
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const int64_t r0 = chunk * MP_ROWS_PER_CHUNK;
         const int64_t r1 = r0 + MP_ROWS_PER_CHUNK < rows ? r0 + MP_ROWS_PER_CHUNK : rows;
         float sum = 0.0f;
+        // Bound by the rows' latency (a column's sum is one chain over its
+        // chunk): sixteen reads in flight.
+#pragma unroll 16
         for (int64_t r = r0; r < r1; ++r) sum += x[r * ld + j];
         partial[chunk * n + j] = sum;
     }
