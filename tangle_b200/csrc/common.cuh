@@ -79,8 +79,8 @@ __device__ inline float reciprocal_plain(float b) {
     return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
 }
 
-// RN(a / b) from y = RN(1 / b), for |a| and b in [PLAIN_MIN, PLAIN_MAX]
-// (a = +0 too): the division by a correctly rounded reciprocal of
+// RN(a / b) from y = RN(1 / b), for |a|, b in [PLAIN_MIN, PLAIN_MAX] and a
+// quotient in [2^-120, 2^120] (a = +0 too): the division by a correctly rounded reciprocal of
 // P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Dev. 34 (1990). The first correction
 // makes q faithful, so the second residual a - b q is exact and the last FMA
