@@ -242,6 +242,16 @@ __device__ inline bool minimum_image(float p1x, float p1y, float p1z, float q1x,
     return moved;
 }
 
+// The closest-point solve's second clamp (neighbor.rs:66-78,
+// contact.rs:683-694): t from the projection on the second axis; where that
+// is past an end, s is solved again at the end (one division for both ends,
+// so that a warp with lanes past either takes it once).
+__device__ inline float keep_on_segment(float projected, float a, float b, float c, float &s) {
+    const bool before = projected < 0.0f, after = projected > 1.0f;
+    if (before || after) s = clampf((before ? -c : b - c) / a, 0.0f, 1.0f);
+    return before ? 0.0f : after ? 1.0f : projected;
+}
+
 // neighbor.rs:27-86 with one proxy piece per segment (the canonical-pair
 // test always passes): distance between the two segment axes.
 __device__ inline float axis_distance(float p1x, float p1y, float p1z, float d1x, float d1y, float d1z,
@@ -265,14 +275,7 @@ __device__ inline float axis_distance(float p1x, float p1y, float p1z, float d1x
             if (fabsf(denominator) > parallel_relative_epsilon * a * e)
                 s = clampf((b * f - c * e) / denominator, 0.0f, 1.0f);
             float projected = (b * s + f) / e;
-            if (projected < 0.0f) {
-                s = clampf(-c / a, 0.0f, 1.0f);
-            } else if (projected > 1.0f) {
-                t = 1.0f;
-                s = clampf((b - c) / a, 0.0f, 1.0f);
-            } else {
-                t = projected;
-            }
+            t = keep_on_segment(projected, a, b, c, s);
         }
     }
     float dx = (p2x + d2x * t) - (p1x + d1x * s);

@@ -141,25 +141,10 @@ __device__ inline bool contact_solve(const Home &h, uint32_t other, float other_
             bool parallel = fabsf(denominator) <= parallel_relative_epsilon * a * e;
             if (!parallel) s = clampf((b * f - c * e) / denominator, 0.0f, 1.0f);
             float projected = (b * s + f) / e;
-            if (projected < 0.0f) {
-                s = clampf(-c / a, 0.0f, 1.0f);
-            } else if (projected > 1.0f) {
-                t = 1.0f;
-                s = clampf((b - c) / a, 0.0f, 1.0f);
-            } else {
-                t = projected;
-            }
+            t = keep_on_segment(projected, a, b, c, s);
             if (parallel) {  // contact.rs:695-726
-                float end_s = 1.0f, end_t = 0.0f;
-                float end_projected = (b + f) / e;
-                if (end_projected < 0.0f) {
-                    end_s = clampf(-c / a, 0.0f, 1.0f);
-                } else if (end_projected > 1.0f) {
-                    end_t = 1.0f;
-                    end_s = clampf((b - c) / a, 0.0f, 1.0f);
-                } else {
-                    end_t = end_projected;
-                }
+                float end_s = 1.0f;
+                const float end_t = keep_on_segment((b + f) / e, a, b, c, end_s);
                 float gx = rx + d1x * s - d2x * t, gy = ry + d1y * s - d2y * t, gz = rz + d1z * s - d2z * t;
                 float ex = rx + d1x * end_s - d2x * end_t, ey = ry + d1y * end_s - d2y * end_t,
                       ez = rz + d1z * end_s - d2z * end_t;
