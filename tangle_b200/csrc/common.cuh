@@ -23,7 +23,7 @@ struct Grid {
     float upper[3];
     float length[3];
     float width[3];
-    float inv_length[3];  // 1 / length in f32, for image_round's fast path
+    float inv_length[3];  // 1 / length in f32, for minimum_image's fast path
     uint32_t periodic[3];
     uint32_t cells[3];
 };
@@ -191,55 +191,53 @@ __device__ inline uint32_t stencil_cell(uint32_t home, uint32_t neighbor, const 
     return (nz * g.cells[1] + ny) * g.cells[0] + nx;
 }
 
-// roundf(x / length[a]) -- the image count of a periodic axis -- without the
-// IEEE division in all but a vanishing set of cases. With q = x * (1/length)
-// rounded twice in f32, |q - x/length| <= |q| 2^-22 and the correctly
-// rounded quotient is within |q| 2^-24 of x/length; for |q| < 4096 both lie
-// within 7.4e-4 of q. Rounding to the nearest integer only changes at
-// half-integers, so when q is more than 1e-3 from one, roundf(q) is exactly
-// roundf(x / length) (same integer, same sign of zero). Otherwise the
-// division is done.
-__device__ inline float image_round(float x, int a, const Grid &g) {
-    float q = x * g.inv_length[a];
-    float aq = fabsf(q);
-    if (aq < 0.499f) return copysignf(0.0f, q);  // the common case: same cell image
-    float fraction = aq - floorf(aq);
-    if (aq < 4096.0f && fabsf(fraction - 0.5f) > 1.0e-3f) return roundf(q);
-    return roundf(x / g.length[a]);
-}
-
 // Minimum-image shift of the second segment against the first, per periodic
-// axis (neighbor.rs:301-318, contact.rs:456-473). Returns true when some axis
-// shifted by a nonzero number of box lengths.
+// axis (neighbor.rs:301-318, contact.rs:456-473): roundf(x / length) box
+// lengths. Returns true when some axis shifted by a nonzero number of them.
+//
+// The image counts come without the IEEE division in all but a vanishing set
+// of cases. With q = x * (1/length) rounded twice in f32, |q - x/length| <=
+// |q| 2^-22 and the correctly rounded quotient is within |q| 2^-24 of
+// x/length; for |q| < 4096 both lie within 7.4e-4 of q. Rounding to the
+// nearest integer only changes at half-integers, so when q is more than 1e-3
+// from one, rintf(q) is exactly roundf(x / length) (same integer, same sign
+// of zero). Where some axis is nearer to one, all three divide. One test for
+// the three axes, as most candidates of an unwrapped fiber sit in another
+// image on one of them, against a branch for the home image and one for the
+// others on each: contact stage of 128 iterations of 2.0 M segments 90.7 ->
+// 86.0 ms, of 48 specimens 32.4 -> 30.9 ms.
 __device__ inline bool minimum_image(float p1x, float p1y, float p1z, float q1x, float q1y, float q1z,
                                      float &p2x, float &p2y, float &p2z, float &q2x, float &q2y, float &q2z,
                                      const Grid &g) {
-    float image_dx = 0.5f * (p2x + q2x - p1x - q1x);
-    float image_dy = 0.5f * (p2y + q2y - p1y - q1y);
-    float image_dz = 0.5f * (p2z + q2z - p1z - q1z);
-    bool moved = false;
+    const float d[3] = {0.5f * (p2x + q2x - p1x - q1x), 0.5f * (p2y + q2y - p1y - q1y), 0.5f * (p2z + q2z - p1z - q1z)};
+    float images[3] = {0.0f, 0.0f, 0.0f};
+    bool sure = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (g.periodic[a]) {
+            const float q = d[a] * g.inv_length[a];
+            images[a] = rintf(q);
+            sure = sure && fabsf(q - images[a]) < 0.499f && fabsf(q) < 4096.0f;
+        }
+    if (!sure)
+        for (int a = 0; a < 3; ++a)
+            if (g.periodic[a]) images[a] = roundf(d[a] / g.length[a]);
     if (g.periodic[0]) {
-        float images = image_round(image_dx, 0, g);
-        float shift = images * g.length[0];
+        const float shift = images[0] * g.length[0];
         p2x -= shift;
         q2x -= shift;
-        moved |= images != 0.0f;
     }
     if (g.periodic[1]) {
-        float images = image_round(image_dy, 1, g);
-        float shift = images * g.length[1];
+        const float shift = images[1] * g.length[1];
         p2y -= shift;
         q2y -= shift;
-        moved |= images != 0.0f;
     }
     if (g.periodic[2]) {
-        float images = image_round(image_dz, 2, g);
-        float shift = images * g.length[2];
+        const float shift = images[2] * g.length[2];
         p2z -= shift;
         q2z -= shift;
-        moved |= images != 0.0f;
     }
-    return moved;
+    return images[0] != 0.0f || images[1] != 0.0f || images[2] != 0.0f;
 }
 
 // The closest-point solve's second clamp (neighbor.rs:66-78,

@@ -470,7 +470,7 @@ __global__ void rb_boxes_kernel(WorldDev w) {
 // the exact test 32 at a time; the lists are sorted later. Rebuild stage per
 // image rounding in every test and a round per cell -> this: 2.0 M segments
 // at 113 per cell 12.1 -> 10.6 ms; 48 specimens (64 iterations) 42.4 -> 35.6
-// ms, where cells hold a dozen and joining them fills the rounds.
+// ms (there every test also read the lengths from memory).
 //
 // Stencil-cell culling (with the sphere test on). rb_boxes_kernel bounds each
 // cell's spheres, radii scaled by 1.0003, by a box in that cell's own frame
