@@ -73,18 +73,17 @@ __device__ inline bool contact_reach_wide(const Home &h, float4 oa, float4 ob, c
     return m2 <= wide * wide;
 }
 
-// Whether two segments (the second already at its minimum image) may come
-// within `extra` of touching: their f32 closest-point distance against
-// r1 + r2 + extra with margins for its rounding. The closest-point solve
-// returns a distance between two points of the segments, so it can only
-// overestimate the true distance, by rounding, or, for axes within 1e-3 rad
-// of parallel (where it takes an end point without solving), by at most
-// 1e-3 of a segment length; the margins (1 % relative, 2e-3 of the summed
-// half lengths, and `eps`) cover both.
-__device__ inline bool within_contact_skin(const Home &h, float p2x, float p2y, float p2z, float q2x, float q2y,
-                                           float q2z, float other_radius, float extra, float eps) {
+// Whether two segments (the second already at its minimum image), with
+// closest points `distance` apart by the solve below, may come within
+// `extra` of touching: that distance against r1 + r2 + extra with margins for
+// its rounding. The solve returns a distance between two points of the
+// segments, so it can only overestimate the true distance, by rounding, or,
+// for axes within 1e-3 rad of parallel (where it takes an end point without
+// solving), by at most 1e-3 of a segment length; the margins (1 % relative,
+// 2e-3 of the summed half lengths, and `eps`) cover both.
+__device__ inline bool within_contact_skin(const Home &h, float distance, float p2x, float p2y, float p2z, float q2x,
+                                           float q2y, float q2z, float other_radius, float extra, float eps) {
     const float d2x = q2x - p2x, d2y = q2y - p2y, d2z = q2z - p2z;
-    const float distance = axis_distance(h.p1x, h.p1y, h.p1z, h.d1x, h.d1y, h.d1z, p2x, p2y, p2z, d2x, d2y, d2z);
     const float other_half = 0.5f * sqrtf(d2x * d2x + d2y * d2y + d2z * d2z);
     const float threshold =
         (h.radius + other_radius + extra) * 1.01f + 2.0e-3f * (h.half_length + other_half) + eps;
@@ -113,16 +112,22 @@ __device__ inline bool lines_may_touch(const Home &h, float p2x, float p2y, floa
     return rn * rn <= threshold * threshold * nn;
 }
 
+// The closest points of a home segment's axis and a candidate's: their
+// parameters, separation and distance.
+struct Closest {
+    float s, t, dx, dy, dz, distance;
+};
+
 // One candidate of find_segment_corrections past the midpoint reject
-// (contact.rs:663-870) for a round lane at zero offset: returns true with
-// the pair's terms when the capsules overlap.
-__device__ inline bool contact_solve(const Home &h, uint32_t other, float other_radius, float p2x, float p2y,
-                                     float p2z, float q2x, float q2y, float q2z, float correction_fraction,
-                                     uint32_t aggregation, PairTerms &out) {
+// (contact.rs:663-870) for a round lane at zero offset, in two parts: the
+// closest points, and from them the pair's terms when the capsules overlap.
+// (A refresh pass decides by the same distance whether to keep the entry;
+// solving a second time for that cost 4 % of the contact stage: 86.0 -> 82.8
+// ms on 128 iterations of 2.0 M segments, 28 of them refreshes.)
+__device__ inline Closest closest_points(const Home &h, float p2x, float p2y, float p2z, float q2x, float q2y, float q2z) {
     const float length_epsilon = 1.0e-20f;
     const float parallel_relative_epsilon = 1.0e-6f;
     const float p1x = h.p1x, p1y = h.p1y, p1z = h.p1z, d1x = h.d1x, d1y = h.d1y, d1z = h.d1z;
-    const float radius = h.radius;
     float d2x = q2x - p2x, d2y = q2y - p2y, d2z = q2z - p2z;
     float rx = p1x - p2x, ry = p1y - p2y, rz = p1z - p2z;
     float a = d1x * d1x + d1y * d1y + d1z * d1z;
@@ -158,16 +163,24 @@ __device__ inline bool contact_solve(const Home &h, uint32_t other, float other_
     float point1x = p1x + d1x * s, point1y = p1y + d1y * s, point1z = p1z + d1z * s;
     float point2x = p2x + d2x * t, point2y = p2y + d2y * t, point2z = p2z + d2z * t;
     float delta_x = point2x - point1x, delta_y = point2y - point1y, delta_z = point2z - point1z;
-    float distance = sqrtf(delta_x * delta_x + delta_y * delta_y + delta_z * delta_z);
-    float penetration = radius + other_radius - distance;
+    return {s, t, delta_x, delta_y, delta_z, sqrtf(delta_x * delta_x + delta_y * delta_y + delta_z * delta_z)};
+}
+
+__device__ inline bool contact_terms(const Home &h, const Closest &at, uint32_t other, float other_radius, float p2x,
+                                     float p2y, float p2z, float q2x, float q2y, float q2z, float correction_fraction,
+                                     uint32_t aggregation, PairTerms &out) {
+    const float s = at.s, t = at.t, distance = at.distance;
+    float penetration = h.radius + other_radius - distance;
     if (!(penetration > 0.0f)) return false;
     float nx, ny, nz;
     if (distance > 1.0e-7f) {
         float inverse_distance = 1.0f / distance;
-        nx = delta_x * inverse_distance;
-        ny = delta_y * inverse_distance;
-        nz = delta_z * inverse_distance;
+        nx = at.dx * inverse_distance;
+        ny = at.dy * inverse_distance;
+        nz = at.dz * inverse_distance;
     } else {  // contact.rs:768-812
+        const float d1x = h.d1x, d1y = h.d1y, d1z = h.d1z;
+        const float d2x = q2x - p2x, d2y = q2y - p2y, d2z = q2z - p2z;
         nx = d1y * d2z - d1z * d2y;
         ny = d1z * d2x - d1x * d2z;
         nz = d1x * d2y - d1y * d2x;
@@ -228,6 +241,13 @@ __device__ inline bool contact_solve(const Home &h, uint32_t other, float other_
     out.t1z = nz * magnitude * weight_1 * aggregate_weight;
     out.aggw = aggregate_weight;
     return true;
+}
+
+__device__ inline bool contact_solve(const Home &h, uint32_t other, float other_radius, float p2x, float p2y,
+                                     float p2z, float q2x, float q2y, float q2z, float correction_fraction,
+                                     uint32_t aggregation, PairTerms &out) {
+    return contact_terms(h, closest_points(h, p2x, p2y, p2z, q2x, q2y, q2z), other, other_radius, p2x, p2y, p2z, q2x, q2y,
+                         q2z, correction_fraction, aggregation, out);
 }
 
 struct ContactAcc {

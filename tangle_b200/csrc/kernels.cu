@@ -1115,11 +1115,12 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
                     const float4 ea = qg[2 * lane], eb = qg[2 * lane + 1];
                     h = qo[lane] & 31;
                     const Home home = make_home(hg[2 * h], hg[2 * h + 1], seg_of[h]);
+                    const Closest at = closest_points(home, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z);
                     if (MODE != CONTACT_REFRESH || (qo[lane] & 0x80))
-                        hit = contact_solve(home, __float_as_uint(eb.w), ea.w, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z,
+                        hit = contact_terms(home, at, __float_as_uint(eb.w), ea.w, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z,
                                             sp.correction_fraction, sp.contact_aggregation, pt);
                     if (MODE == CONTACT_REFRESH)
-                        keep = within_contact_skin(home, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z, ea.w,
+                        keep = within_contact_skin(home, at.distance, ea.x, ea.y, ea.z, eb.x, eb.y, eb.z, ea.w,
                                                    A ? lane_skin[A && MODE == CONTACT_REFRESH ? warp : 0][h] : cskin_world,
                                                    A ? w.specs[lane_spec[A ? warp : 0][h]].line_eps : line_eps_world);
                 }
