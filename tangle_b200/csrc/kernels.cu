@@ -7,14 +7,15 @@
 //   contact_kernel    find_segment_corrections (contact.rs:232-902); the
 //                     last block to finish reduces the gate metrics and runs
 //                     assess_reduced_metrics (kernels.rs:129-162)
-//   fiber_kernel      everything after the gate, which only ever touches one
+//   fiber_lanes_kernel everything after the gate, which only ever touches one
 //                     fiber: internal stretch/bend x constraint_iterations
 //                     (kernels.rs:1027-1163, :1417-1453), apply contact
 //                     (:1455-1537), curvature Gauss-Seidel (:1165-1415), the
 //                     displacement check (neighbor.rs:446-465) and the next
 //                     gate's curvature and step measurements (:925-980,
-//                     :95-127). One warp owns one fiber, staged in shared
-//                     memory.
+//                     :95-127), on fibers staged in shared memory, 4 to 32
+//                     lanes each in the sweeps (fiber_kernel: fibers of more
+//                     than 930 vertices, one warp each)
 // Float reductions that feed positions are done in the reference's order
 // (contacts summed in ascending list order); only maxima, which are exact in
 // any order, use atomics (on u32 bits of non-negative floats).
@@ -910,7 +911,8 @@ enum { CONTACT_FULL = 0, CONTACT_REFRESH = 1, CONTACT_LISTED = 2 };
 // specimen: grid and line margin for its candidates, whether the specimen is
 // still active, and the specimen whose gate its penetration feeds.
 template <int MODE, bool A = false>
-__global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams sp, int gate, float line_eps_world) {
+__global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams sp, int gate, float line_eps_world,
+                                                         int split_shift) {
     __shared__ float4 home_geom[CONTACT_WARPS][64];
     __shared__ uint32_t prefix[CONTACT_WARPS][33];
     __shared__ float4 queue_geom[CONTACT_WARPS][128];  // 64 entries: {p2, r2}, {q2, other}
@@ -964,14 +966,19 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
     // queue on the counter's one address (measured on 512 specimens: 4.26 ms
     // per pass with the counter against 2.47 ms with the stride, while one
     // mid-size world's 62 k batches run 0.283 ms against 0.309 ms).
-    const auto take_batch = [&]() {
+    // A batch's segments may go to 1 << split_shift warps (not in an arena or
+    // a refresh, whose warp writes the batch's whole chunk): see plan_launches.
+    const auto take_part = [&]() {
         uint32_t b = 0;
         if (lane == 0) b = atomicAdd(&w.ctl->next_batch, 1u);
-        return __shfl_sync(FULL, b, 0) * 32u;
+        return __shfl_sync(FULL, b, 0);
     };
-    const uint32_t stride = gridDim.x * CONTACT_WARPS * 32u;
-    for (uint32_t base = A ? (blockIdx.x * CONTACT_WARPS + warp) * 32u : take_batch(); base < w.NS;
-         base = A ? base + stride : take_batch()) {
+    const uint32_t shift = A || MODE == CONTACT_REFRESH ? 0u : (uint32_t)split_shift;
+    const uint32_t parts = ((w.NS + 31u) / 32u) << shift, stride = gridDim.x * CONTACT_WARPS;
+    for (uint32_t part = A ? blockIdx.x * CONTACT_WARPS + warp : take_part(); part < parts;
+         part = A ? part + stride : take_part()) {
+        const uint32_t base = (part >> shift) * 32u;
+        const bool mine = (uint32_t)lane >> (5u - shift) == (part & ((1u << shift) - 1u));
         // Batches follow the cell list's slot order, so the 32 segments of a
         // batch are spatial neighbors and share most of their candidates.
         const bool in_range = base + lane < w.NS;
@@ -980,7 +987,7 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
         // Segments of an arena specimen whose gate has stopped it are
         // skipped; of the others, a listed pass takes those whose specimen's
         // lists hold and a refresh pass those whose specimen's flag is up.
-        const bool alive = in_range && (!A || ctl_of<A>(w, my_spec)->control[0] != 0);
+        const bool alive = in_range && mine && (!A || ctl_of<A>(w, my_spec)->control[0] != 0);
         const bool flagged = A && MODE != CONTACT_FULL && alive && ctl_of<A>(w, my_spec)->contact_state[0] != 0;
         const bool valid = MODE == CONTACT_LISTED ? alive && !flagged : MODE == CONTACT_REFRESH && A ? flagged : alive;
         // A listed pass reads the slot's contact-list state (coalesced), and
@@ -2688,7 +2695,16 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     // Three 256-thread blocks are resident per SM at the kernel's launch
     // bounds; fewer leave room to the kernels around it.
     const int contact_per_sm = lp.tune_contact_per_sm >= 1 && lp.tune_contact_per_sm <= 3 ? lp.tune_contact_per_sm : 3;
-    lp.contact_blocks = grid_for((w.NS + 31) / 32, CONTACT_WARPS, lp.num_sms * contact_per_sm);
+    const uint32_t batches = (w.NS + 31) / 32, resident = (uint32_t)(lp.num_sms * contact_per_sm) * CONTACT_WARPS;
+    // Four warps share a batch's segments while each batch could have a warp
+    // of its own (a warp's chain of rounds is then the pass): contact stage of
+    // 40 31-vertex fibers 2.44 -> 2.22 ms per 128 iterations, of 357-vertex
+    // ones 2.61 -> 2.37, of 886 of 66 and 180 4.51 -> 4.33. With 1.7 batches a
+    // warp or more, the fuller rounds of whole batches win: 6.21 ms against
+    // 7.69 with four and 6.58 with two (2,000 of 108, relaxed).
+    lp.contact_split = !lp.arena && batches <= resident ? 2 : 0;
+    lp.contact_unsplit = grid_for(batches, CONTACT_WARPS, lp.num_sms * contact_per_sm);
+    lp.contact_blocks = grid_for((uint64_t)batches << lp.contact_split, CONTACT_WARPS, lp.num_sms * contact_per_sm);
     // Update kernel: as many warps per block as fit 96 KB of staged fibers.
     size_t per_warp = (size_t)3 * w.max_fiber * sizeof(float4);
     int warps = 8;
@@ -2702,7 +2718,9 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     // By default a warp per fiber while all of those warps are resident at
     // once (the sweeps' chains then take all the lanes there are), and a
     // quarter warp where the chip is full without (four fibers share each
-    // round's instructions).
+    // round's instructions). Update of a batch with 32 lanes and with 8: 40
+    // fibers 7.9 and 9.7 ms, 886 25.9 and 31.4, 2,000 7.7 and 9.7; 4,999
+    // 11.0 and 9.2, 20,000 90.7 and 56.2.
     lp.lanes_per_fiber = w.FA <= (uint32_t)lp.num_sms * 16u ? 32 : 8;
     if (const char *env = std::getenv("TGL_LANES_PER_FIBER")) lp.lanes_per_fiber = std::atoi(env);
     if (lp.tune_lanes) lp.lanes_per_fiber = lp.tune_lanes;
@@ -2714,11 +2732,9 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     lp.lanes_stride = (int)(w.max_fiber | 1u);
     lp.lanes_smem = (size_t)2 * fpw * lp.lanes_stride * sizeof(float4);
     lp.fiber_lanes = (int)w.max_fiber - 2 <= 32 * STRIP_MAX && lp.lanes_smem <= 200 * 1024;
-    // Warps per block: 4 where their staged fibers fit, so that 32 warps
-    // (the register file at the kernel's 64 registers, and 8 blocks of 4
-    // warps) are resident per SM instead of the 28 that one-warp blocks get
-    // (their shared memory and 1 KB reserve per block run out first); the
-    // long tail of the grid then runs on a full SM.
+    // Warps per block: 4 where their staged fibers fit, under one block's
+    // shared-memory reserve (update of 4,999 fibers 9.2 ms, 9.8 with one-warp
+    // blocks and 10.0 with two; of 20,000 56.2, 57.4 and 55.9 ms).
     const int wpb_max = lp.tune_wpb == 1 || lp.tune_wpb == 2 ? lp.tune_wpb : 4;
     lp.lanes_wpb = 1;
     while (lp.lanes_wpb < wpb_max && lp.lanes_smem * (size_t)(2 * lp.lanes_wpb) <= 200 * 1024) lp.lanes_wpb *= 2;
@@ -2876,21 +2892,22 @@ int launch_step_condition(const WorldDev &w, cudaGraphConditionalHandle rebuild,
 int launch_contact(const WorldDev &w, const LaunchPlan &lp, const StepParams &sp, bool gate, cudaStream_t st) {
     if (lp.arena) {
         if (gate && lp.contact_lists) {
-            contact_kernel<CONTACT_LISTED, true><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps);
-            contact_kernel<CONTACT_REFRESH, true><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps);
+            contact_kernel<CONTACT_LISTED, true><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps, 0);
+            contact_kernel<CONTACT_REFRESH, true><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps, 0);
             return 2;
         }
         contact_kernel<CONTACT_FULL, true><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, gate ? 1 : 0,
-                                                                                            lp.line_eps);
+                                                                                            lp.line_eps, 0);
         return 1;
     }
     if (gate && lp.contact_lists) {
         // Listed first: the refresh pass clears the flag the listed pass reads.
-        contact_kernel<CONTACT_LISTED><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps);
-        contact_kernel<CONTACT_REFRESH><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps);
+        contact_kernel<CONTACT_LISTED><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps, lp.contact_split);
+        contact_kernel<CONTACT_REFRESH><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, 1, lp.line_eps, 0);
         return 2;
     }
-    contact_kernel<CONTACT_FULL><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, gate ? 1 : 0, lp.line_eps);
+    contact_kernel<CONTACT_FULL><<<lp.contact_blocks, CONTACT_WARPS * 32, 0, st>>>(w, sp, gate ? 1 : 0, lp.line_eps,
+                                                                                    lp.contact_split);
     return 1;
 }
 

@@ -222,6 +222,8 @@ struct LaunchPlan {
     int num_sms;
     int contact_group;      // lanes per segment in the contact pass (8, 16 or 32)
     int contact_blocks;
+    int contact_split;      // log2 of the warps that share a contact batch
+    int contact_unsplit;    // contact_blocks if none were shared (reported)
     float line_eps;         // absolute margin of the contact pass's line-distance bound
     int fiber_warps;        // fibers per block of the update kernel
     int fiber_blocks;

@@ -1847,7 +1847,7 @@ int check_launch_params(const tgl_world *w, const tgl_launch_params &p) {
 void current_launch_params(const tgl_world *w, tgl_launch_params *p) {
     std::memset(p, 0, sizeof(*p));
     p->lanes_per_fiber = (uint32_t)w->lp.lanes_per_fiber;
-    const int per_sm = (w->lp.contact_blocks + w->lp.num_sms - 1) / std::max(w->lp.num_sms, 1);
+    const int per_sm = (w->lp.contact_unsplit + w->lp.num_sms - 1) / std::max(w->lp.num_sms, 1);
     p->contact_blocks_per_sm = (uint32_t)(w->lp.tune_contact_per_sm ? w->lp.tune_contact_per_sm : std::min(3, std::max(per_sm, 1)));
     p->build_chunk = (uint32_t)w->lp.build_ch;
     p->contact_skin_fraction = w->contact_fraction;
