@@ -188,6 +188,9 @@ class ContactGraph:
             edges = ctypes.c_int64()
             _check(lib.tgl_warmstart_graph_count(world._handle, ctypes.c_float(cutoff), ctypes.byref(edges)))
             g = cls(world.vertex_count, world.segment_count, int(edges.value), torch.device("cuda"))
+            # The world fills them on its own stream: not before the kernels
+            # that torch's stream was given over the same (reused) memory.
+            torch.cuda.ExternalStream(world.stream_handle).wait_stream(torch.cuda.current_stream())
             out = _MpGraphOut(_p(g.seg_v0), _p(g.links), _p(g.offsets), _p(g.dst), _p(g.src), _p(g.twin), _p(g.s),
                               _p(g.t), _p(g.node_features), _p(g.edge_features))
             _check(lib.tgl_warmstart_graph_fill(world._handle, ctypes.byref(out)))
