@@ -1863,11 +1863,11 @@ int apply_launch_params(tgl_world *w, const tgl_launch_params &p) {
     if (w->dev.contact_block) set_contact_skin(w, p.contact_skin_fraction);
     plan_launches(w->dev, w->lp);
     drop_graphs(w);
-    // The contact lists were filtered at the old skin: refresh them first.
+    // The contact lists were filtered at the old skin: refresh them first, in
+    // an arena every specimen's (the flags are 0, 1 or 2: their low byte).
     if (w->dev.contact_block) {
-        const uint32_t one = 1;
-        TGL_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(w->dev.ctl) + offsetof(Control, contact_state), &one,
-                                 sizeof(uint32_t), cudaMemcpyHostToDevice, w->stream));
+        TGL_CUDA(cudaMemset2DAsync(reinterpret_cast<char *>(w->dev.ctl) + offsetof(Control, contact_state),
+                                   sizeof(Control), 1, 1, w->arena ? w->specimens + 1 : 1, w->stream));
         TGL_CUDA(cudaStreamSynchronize(w->stream));
     }
     return 0;
