@@ -670,6 +670,7 @@ int prepare_specimen(const tgl_packed *pk, const tgl_cell_list_config *cl, float
 namespace {
 
 void set_contact_skin(tgl_world *w, float fraction);
+bool bound_contact_lists(tgl_world *w);
 
 // Device world from prepared specimens: one (a single world) or several (an
 // arena, relaxed together with a gate per specimen).
@@ -1692,14 +1693,7 @@ int tgl_world_compact_cell(tgl_world *w, const float new_lower[3], const float n
     d.C = (uint32_t)C;
     w->contact_grids.assign(1, d.grid);
     // The contact lists' single-image bound follows the new box edges.
-    if (d.contact_skin > 0.0f) {
-        d.contact_half_limit = INFINITY;
-        for (int a = 0; a < 3; ++a)
-            if (d.grid.periodic[a])
-                d.contact_half_limit =
-                    std::fmin(d.contact_half_limit,
-                              0.999f * 0.5f * (0.5f * d.grid.length[a] - 2.0f * w->maximum_radius - d.contact_wide));
-    }
+    if (d.contact_skin > 0.0f) bound_contact_lists(w);
     plan_launches(d, w->lp);
     w->launches += launch_refresh_geometry(d, w->stream);
     w->launches += launch_request_rebuild(d, w->lp, w->stream);  // world.rs:2052
@@ -1796,29 +1790,37 @@ int tgl_world_set_fiber_max_curvatures(tgl_world *w, const float *values, size_t
 
 namespace {
 
-// The contact skin and its single-image bound for a fraction of the
-// neighbor skin (as build_world sets them); a fraction the bound leaves no
-// room for turns the lists off.
-void set_contact_skin(tgl_world *w, float fraction) {
+// The wide contact skin and the single-image bound of the contact lists. A
+// pair's minimum image must stay fixed while its vertices move less than the
+// lists' skin: with every half length below H, pairs within reach + skin are
+// closer than half a box length on every periodic axis, so
+// H = (L/2 - 2 r_max - skin) / 2, less 0.1 %, over every specimen's box. The
+// skin is the wide one (2.5 times the narrow, at most the neighbor skin)
+// where that leaves room for the longest segment, else the narrow one; false
+// when that leaves none either, and every pass is a refresh while some
+// segment is too long.
+bool bound_contact_lists(tgl_world *w) {
     WorldDev &d = w->dev;
-    d.contact_skin = fraction > 0.0f ? fraction * w->contact_skin_base : 0.0f;
-    // A pair's minimum image must stay fixed while its vertices move less
-    // than the contact skin: with every half length below H, pairs within
-    // reach + contact skin are closer than half a box length on every
-    // periodic axis, so H = (L/2 - 2 r_max - contact_skin) / 2, less 0.1 %,
-    // over every specimen's box. The wide skin where it leaves room.
-    d.contact_wide = std::fmin(2.5f * d.contact_skin, std::fmax(w->contact_skin_base, d.contact_skin));
-    for (int attempt = 0; attempt < 2; ++attempt) {
+    const float wide = std::fmin(2.5f * d.contact_skin, std::fmax(w->contact_skin_base, d.contact_skin));
+    for (const float skin : {wide, d.contact_skin}) {
+        d.contact_wide = skin;
         d.contact_half_limit = INFINITY;
         for (const Grid &g : w->contact_grids)
             for (int a = 0; a < 3; ++a)
                 if (g.periodic[a])
-                    d.contact_half_limit = std::fmin(
-                        d.contact_half_limit, 0.999f * 0.5f * (0.5f * g.length[a] - 2.0f * w->maximum_radius - d.contact_wide));
-        if (d.contact_half_limit > 0.5f * w->maximum_length) break;
-        d.contact_wide = d.contact_skin;
+                    d.contact_half_limit = std::fmin(d.contact_half_limit,
+                                                     0.999f * 0.5f * (0.5f * g.length[a] - 2.0f * w->maximum_radius - skin));
+        if (d.contact_half_limit > 0.5f * w->maximum_length) return true;
     }
-    if (!(d.contact_half_limit > 0.5f * w->maximum_length)) d.contact_skin = 0.0f;  // no room: full lists every pass
+    return false;
+}
+
+// The contact skin and its bound for a fraction of the neighbor skin; a
+// fraction that the bound leaves no room for turns the lists off.
+void set_contact_skin(tgl_world *w, float fraction) {
+    WorldDev &d = w->dev;
+    d.contact_skin = fraction > 0.0f ? fraction * w->contact_skin_base : 0.0f;
+    if (!bound_contact_lists(w)) d.contact_skin = 0.0f;  // no room: full lists every pass
     w->contact_fraction = d.contact_skin > 0.0f ? fraction : 0.0f;
 }
 
