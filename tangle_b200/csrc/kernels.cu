@@ -2678,6 +2678,18 @@ static void allow_dynamic_smem(Kernel kernel, size_t bytes) {
         current = bytes;
 }
 
+void plan_contact_pass(const WorldDev &w, LaunchPlan &lp, int per_sm) {
+    const uint32_t batches = (w.NS + 31) / 32, resident = (uint32_t)(lp.num_sms * per_sm) * CONTACT_WARPS;
+    // Four warps share a batch's segments while each batch could have a warp
+    // of its own (a warp's chain of rounds is then the pass): contact stage of
+    // 40 31-vertex fibers 2.44 -> 2.22 ms per 128 iterations, of 357-vertex
+    // ones 2.61 -> 2.37, of 886 of 66 and 180 4.51 -> 4.33. With 1.7 batches a
+    // warp or more, the fuller rounds of whole batches win: 6.21 ms against
+    // 7.69 with four and 6.58 with two (2,000 of 108, relaxed).
+    lp.contact_split = !lp.arena && batches <= resident ? 2 : 0;
+    lp.contact_blocks = grid_for((uint64_t)batches << lp.contact_split, CONTACT_WARPS, lp.num_sms * per_sm);
+}
+
 void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     int device = 0;
     cudaGetDevice(&device);
@@ -2695,16 +2707,7 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     // Three 256-thread blocks are resident per SM at the kernel's launch
     // bounds; fewer leave room to the kernels around it.
     const int contact_per_sm = lp.tune_contact_per_sm >= 1 && lp.tune_contact_per_sm <= 3 ? lp.tune_contact_per_sm : 3;
-    const uint32_t batches = (w.NS + 31) / 32, resident = (uint32_t)(lp.num_sms * contact_per_sm) * CONTACT_WARPS;
-    // Four warps share a batch's segments while each batch could have a warp
-    // of its own (a warp's chain of rounds is then the pass): contact stage of
-    // 40 31-vertex fibers 2.44 -> 2.22 ms per 128 iterations, of 357-vertex
-    // ones 2.61 -> 2.37, of 886 of 66 and 180 4.51 -> 4.33. With 1.7 batches a
-    // warp or more, the fuller rounds of whole batches win: 6.21 ms against
-    // 7.69 with four and 6.58 with two (2,000 of 108, relaxed).
-    lp.contact_split = !lp.arena && batches <= resident ? 2 : 0;
-    lp.contact_unsplit = grid_for(batches, CONTACT_WARPS, lp.num_sms * contact_per_sm);
-    lp.contact_blocks = grid_for((uint64_t)batches << lp.contact_split, CONTACT_WARPS, lp.num_sms * contact_per_sm);
+    plan_contact_pass(w, lp, contact_per_sm);
     // Update kernel: as many warps per block as fit 96 KB of staged fibers.
     size_t per_warp = (size_t)3 * w.max_fiber * sizeof(float4);
     int warps = 8;

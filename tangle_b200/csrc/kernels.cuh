@@ -223,7 +223,6 @@ struct LaunchPlan {
     int contact_group;      // lanes per segment in the contact pass (8, 16 or 32)
     int contact_blocks;
     int contact_split;      // log2 of the warps that share a contact batch
-    int contact_unsplit;    // contact_blocks if none were shared (reported)
     float line_eps;         // absolute margin of the contact pass's line-distance bound
     int fiber_warps;        // fibers per block of the update kernel
     int fiber_blocks;
@@ -282,5 +281,7 @@ int launch_positions_to_stage(const WorldDev &w, cudaStream_t st);
 int launch_corrections_to_stage(const WorldDev &w, float *corr6, float *pen, cudaStream_t st);
 
 void plan_launches(const WorldDev &w, LaunchPlan &lp);
+// The contact pass's part of it, for `per_sm` blocks per SM.
+void plan_contact_pass(const WorldDev &w, LaunchPlan &lp, int per_sm);
 
 }  // namespace tgl

@@ -1849,20 +1849,27 @@ int check_launch_params(const tgl_world *w, const tgl_launch_params &p) {
 void current_launch_params(const tgl_world *w, tgl_launch_params *p) {
     std::memset(p, 0, sizeof(*p));
     p->lanes_per_fiber = (uint32_t)w->lp.lanes_per_fiber;
-    const int per_sm = (w->lp.contact_unsplit + w->lp.num_sms - 1) / std::max(w->lp.num_sms, 1);
-    p->contact_blocks_per_sm = (uint32_t)(w->lp.tune_contact_per_sm ? w->lp.tune_contact_per_sm : std::min(3, std::max(per_sm, 1)));
+    // Untuned: the fewest blocks per SM whose plan is the one in use, so that
+    // setting what is reported changes nothing.
+    int per_sm = w->lp.tune_contact_per_sm ? w->lp.tune_contact_per_sm : 1;
+    for (; !w->lp.tune_contact_per_sm && per_sm < 3; ++per_sm) {
+        LaunchPlan same = w->lp;
+        plan_contact_pass(w->dev, same, per_sm);
+        if (same.contact_blocks == w->lp.contact_blocks && same.contact_split == w->lp.contact_split) break;
+    }
+    p->contact_blocks_per_sm = (uint32_t)per_sm;
     p->build_chunk = (uint32_t)w->lp.build_ch;
     p->contact_skin_fraction = w->contact_fraction;
     p->update_warps_per_block = (uint32_t)(w->lp.tune_wpb ? w->lp.tune_wpb : 4);
 }
 
-int apply_launch_params(tgl_world *w, const tgl_launch_params &p) {
-    if (int rc = check_launch_params(w, p)) return rc;
-    w->lp.tune_lanes = (int)p.lanes_per_fiber;
-    w->lp.tune_contact_per_sm = (int)p.contact_blocks_per_sm;
-    w->lp.tune_build_ch = (int)p.build_chunk;
-    w->lp.tune_wpb = (int)p.update_warps_per_block;
-    if (w->dev.contact_block) set_contact_skin(w, p.contact_skin_fraction);
+// Plans the world anew with `tuned`'s launch shapes (0: the planner's own).
+int replan(tgl_world *w, const LaunchPlan &tuned, float contact_skin_fraction) {
+    w->lp.tune_lanes = tuned.tune_lanes;
+    w->lp.tune_contact_per_sm = tuned.tune_contact_per_sm;
+    w->lp.tune_build_ch = tuned.tune_build_ch;
+    w->lp.tune_wpb = tuned.tune_wpb;
+    if (w->dev.contact_block) set_contact_skin(w, contact_skin_fraction);
     plan_launches(w->dev, w->lp);
     drop_graphs(w);
     // The contact lists were filtered at the old skin: refresh them first, in
@@ -1873,6 +1880,16 @@ int apply_launch_params(tgl_world *w, const tgl_launch_params &p) {
         TGL_CUDA(cudaStreamSynchronize(w->stream));
     }
     return 0;
+}
+
+int apply_launch_params(tgl_world *w, const tgl_launch_params &p) {
+    if (int rc = check_launch_params(w, p)) return rc;
+    LaunchPlan tuned = w->lp;
+    tuned.tune_lanes = (int)p.lanes_per_fiber;
+    tuned.tune_contact_per_sm = (int)p.contact_blocks_per_sm;
+    tuned.tune_build_ch = (int)p.build_chunk;
+    tuned.tune_wpb = (int)p.update_warps_per_block;
+    return replan(w, tuned, p.contact_skin_fraction);
 }
 
 // The state a trial batch changes and the search restores: positions, the
@@ -1988,15 +2005,16 @@ int tgl_autotune(tgl_world *w, const tgl_relax_config *config, uint32_t trial_it
     tgl_launch_params current{};
     current_launch_params(w, &current);
     const tgl_launch_params original = current;
+    const LaunchPlan untouched = w->lp;
     float current_ms = INFINITY;
     uint32_t trials = 0;
     auto fail = [&](int rc) {
-        apply_launch_params(w, original);
+        replan(w, untouched, original.contact_skin_fraction);
         restore_state(w, saved);
         if (was_timing) tgl_set_kernel_timing(w, 1);
         return rc;
     };
-    if (int rc = apply_launch_params(w, current)) return fail(rc);
+    // The baseline: the plan as it is.
     if (int rc = trial(w, saved, trial_config, trial_iterations, &current_ms)) return fail(rc);
     ++trials;
     const float default_ms = current_ms;
@@ -2033,7 +2051,9 @@ int tgl_autotune(tgl_world *w, const tgl_relax_config *config, uint32_t trial_it
             }
         }
     }
-    if (int rc = apply_launch_params(w, current)) return fail(rc);
+    const bool kept = std::memcmp(&current, &original, sizeof(current)) == 0;
+    if (int rc = kept ? replan(w, untouched, original.contact_skin_fraction) : apply_launch_params(w, current))
+        return fail(rc);
     if (int rc = restore_state(w, saved)) return fail(rc);
     if (was_timing) tgl_set_kernel_timing(w, 1);
     *best = current;
