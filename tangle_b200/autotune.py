@@ -9,21 +9,26 @@ model and workload shape, so a later world of the same shape applies it
 without searching.
 
 The cache is a JSON file: `TGL_AUTOTUNE_CACHE`, else
-`~/.cache/tangle_b200/autotune.json`. Entries are keyed by the GPU name and
-the world's shape: vertex, segment, fiber and cell counts, the cell grid,
-the neighbor-list block, the number of specimens (arenas), the longest
-fiber and the motion model. The reference has no counterpart (its CubeCL
-kernels take fixed launch shapes).
+`~/.cache/tangle_b200/autotune.json`. Entries are keyed by the GPU name, the
+kernels (a digest of their sources: a shape found on other kernels is no
+guide) and the world's shape: vertex, segment, active fiber and cell counts,
+the cell grid, the neighbor-list block, the number of specimens (arenas), the
+longest fiber and the motion model. The reference has no counterpart (its
+CubeCL kernels take fixed launch shapes).
 """
 
 from __future__ import annotations
 
+import hashlib
 import json
 import os
 import tempfile
 from pathlib import Path
 from typing import Optional
 
+import numpy as np
+
+from . import build
 from .settings import RelaxationConfig
 
 
@@ -48,8 +53,23 @@ def workload_key(gpu: str, shape: dict) -> str:
     return json.dumps({"gpu": gpu, **{k: shape[k] for k in sorted(shape)}}, sort_keys=True)
 
 
+def kernels() -> str:
+    """A digest of the kernels' sources (of the built library where those
+    were not installed)."""
+    sources = build.SOURCES + build.HEADERS
+    digest = hashlib.sha256()
+    for path in sources if all(os.path.exists(p) for p in sources) else [build.LIB]:
+        with open(path, "rb") as fh:
+            digest.update(fh.read())
+    return digest.hexdigest()[:16]
+
+
 def world_shape(world, config: RelaxationConfig) -> dict:
+    active = getattr(world, "fiber_active", None) if getattr(world, "specimen_vertices", None) is None else None
     return {
+        "kernels": kernels(),
+        "active_fibers": world.fiber_count if active is None else int(np.count_nonzero(active)),
+        "longest_fiber": world.longest_fiber,
         "vertices": int(world.vertex_count),
         "segments": int(world.segment_count),
         "cells": int(world.cell_count),

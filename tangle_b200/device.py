@@ -15,7 +15,7 @@ from __future__ import annotations
 import ctypes
 from dataclasses import dataclass
 import os
-from typing import List, Optional
+from typing import List, Optional, Tuple
 
 import numpy as np
 
@@ -383,6 +383,12 @@ class ContactCapture:
     overflow: bool
 
 
+def fiber_lengths(packeds) -> Tuple[int, int]:
+    """The number of fibers of packed assemblies and the most vertices in one."""
+    counts = np.concatenate([np.asarray(p.fiber_vertex_spans).reshape(-1, 2)[:, 1] for p in packeds])
+    return counts.size, int(counts.max(initial=0))
+
+
 class DeviceWorld(FormationHooks):
     """Resident relaxation world on the current CUDA device."""
 
@@ -407,6 +413,7 @@ class DeviceWorld(FormationHooks):
         self._packed = packed
         self.vertex_count = packed.vertex_count
         self.segment_count = packed.segment_count
+        self.fiber_count, self.longest_fiber = fiber_lengths([packed])
         if not np.all(np.asarray(packed.fiber_active)):
             self.set_active_fibers(np.asarray(packed.fiber_active))
 
@@ -435,6 +442,7 @@ class DeviceWorld(FormationHooks):
         world._packed = None
         world.vertex_count = sum(p.vertex_count for p in packeds)
         world.segment_count = sum(p.segment_count for p in packeds)
+        world.fiber_count, world.longest_fiber = fiber_lengths(packeds)
         world.specimen_vertices = [p.vertex_count for p in packeds]
         return world
 
