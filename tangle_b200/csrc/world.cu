@@ -11,7 +11,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/tangle_cuda.h"
@@ -1882,14 +1884,20 @@ int replan(tgl_world *w, const LaunchPlan &tuned, float contact_skin_fraction) {
     return 0;
 }
 
-int apply_launch_params(tgl_world *w, const tgl_launch_params &p) {
-    if (int rc = check_launch_params(w, p)) return rc;
+// The plan that `p` asks for.
+LaunchPlan tuned_plan(const tgl_world *w, const tgl_launch_params &p) {
     LaunchPlan tuned = w->lp;
     tuned.tune_lanes = (int)p.lanes_per_fiber;
     tuned.tune_contact_per_sm = (int)p.contact_blocks_per_sm;
     tuned.tune_build_ch = (int)p.build_chunk;
     tuned.tune_wpb = (int)p.update_warps_per_block;
-    return replan(w, tuned, p.contact_skin_fraction);
+    plan_launches(w->dev, tuned);
+    return tuned;
+}
+
+int apply_launch_params(tgl_world *w, const tgl_launch_params &p) {
+    if (int rc = check_launch_params(w, p)) return rc;
+    return replan(w, tuned_plan(w, p), p.contact_skin_fraction);
 }
 
 // The state a trial batch changes and the search restores: positions, the
@@ -2018,6 +2026,12 @@ int tgl_autotune(tgl_world *w, const tgl_relax_config *config, uint32_t trial_it
     if (int rc = trial(w, saved, trial_config, trial_iterations, &current_ms)) return fail(rc);
     ++trials;
     const float default_ms = current_ms;
+    // What of the parameters a plan's launches depend on: one already timed
+    // is not timed again under another name.
+    const auto launches = [&](const LaunchPlan &lp, float fraction) {
+        return std::make_tuple(lp.strip_lanes, lp.lanes_wpb, lp.contact_blocks, lp.contact_split, lp.build_ch, fraction);
+    };
+    std::set<decltype(launches(untouched, 0.0f))> timed = {launches(untouched, original.contact_skin_fraction)};
     const bool lanes = w->lp.fiber_lanes && config->motion_model == 0;
     const uint32_t lane_choices[] = {2, 4, 8, 32};
     const uint32_t block_choices[] = {1, 2, 3};
@@ -2040,7 +2054,7 @@ int tgl_autotune(tgl_world *w, const tgl_relax_config *config, uint32_t trial_it
         if (parameter == 4 && lanes)
             for (uint32_t v : wpb_choices) c.update_warps_per_block = v, candidates.push_back(c);
         for (const tgl_launch_params &candidate : candidates) {
-            if (std::memcmp(&candidate, &current, sizeof(candidate)) == 0) continue;
+            if (!timed.insert(launches(tuned_plan(w, candidate), candidate.contact_skin_fraction)).second) continue;
             if (int rc = apply_launch_params(w, candidate)) return fail(rc);
             float ms = INFINITY;
             if (int rc = trial(w, saved, trial_config, trial_iterations, &ms)) return fail(rc);
