@@ -2260,13 +2260,16 @@ __global__ void __launch_bounds__(ORDER_THREADS) order_by_rounds_kernel(WorldDev
 // fiber's specimen.
 // FM compiles in the formation work (wall reactions, layer and vertex
 // targets); without it the kernel carries none of it.
-template <int LPF, bool A = false, bool FM = false>
-__global__ void __launch_bounds__(128, A ? 6 : 4) fiber_lanes_kernel(WorldDev w, StepParams sp, int stride) {
+// Without SWEEP (worlds whose longest fiber has two vertices, at eight lanes)
+// half the registers go and twice the warps are resident, whose loads are all
+// the kernel waits for: 64 updates of 200,000 such fibers 13.4 against 19.1 ms.
+template <int LPF, bool A = false, bool FM = false, bool SWEEP = true>
+__global__ void __launch_bounds__(128, !SWEEP ? 8 : A ? 6 : 4) fiber_lanes_kernel(WorldDev w, StepParams sp, int stride) {
     constexpr int FPW = 32 / LPF;  // fibers per warp
     if (w.ctl->control[0] == 0) return;
     extern __shared__ float4 lanes_smem_all[];
     // Each warp works alone on its own fibers; a block holds up to 4 warps
-    // only so that 32 warps fit on an SM (at most 32 blocks are resident).
+    // so that they share one block's shared-memory reserve.
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     // The warp's fibers in one record array, and as much room again; the
@@ -2376,8 +2379,10 @@ __global__ void __launch_bounds__(128, A ? 6 : 4) fiber_lanes_kernel(WorldDev w,
             const bool reacts = FM && mine != TGL_NONE && w.reaction != nullptr;
             float4 *const R = reacts ? w.reaction + w.fiber_vspan[mine].x : nullptr;
             float4 *const R_next = reacts ? w.reaction_next + w.fiber_vspan[mine].x : nullptr;
-            const uint32_t rounds = sweep_curvature<LPF, FM>(staged + (size_t)group * stride, room + (size_t)group * stride,
-                                                             triplets, sp, extent, g, R, R_next);
+            uint32_t rounds = 0;
+            if (SWEEP)
+                rounds = sweep_curvature<LPF, FM>(staged + (size_t)group * stride, room + (size_t)group * stride, triplets, sp,
+                                                  extent, g, R, R_next);
             // The rounds this fiber's sweeps took rank it for the next updates
             // (a fiber of a stopped specimen took none).
             if (!A && w.fiber_rounds != nullptr && mine != TGL_NONE && gl == 0) w.fiber_rounds[mine] = rounds;
@@ -2718,13 +2723,21 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     // Grouped-lane update: an odd float4 stride per fiber so that the groups'
     // same-index accesses spread over the banks. The lanes per fiber asked
     // for are raised until a strip's triplets fit its word.
-    // By default a warp per fiber while all of those warps are resident at
-    // once (the sweeps' chains then take all the lanes there are), and a
-    // quarter warp where the chip is full without (four fibers share each
+    // By default a warp per fiber up to 16 fibers an SM, the warps that the
+    // kernel's registers leave resident (the sweeps' chains then take all the
+    // lanes there are; fibers past about 250 vertices leave fewer, by their
+    // staged records), and a quarter warp beyond (four fibers share each
     // round's instructions). Update of a batch with 32 lanes and with 8: 40
     // fibers 7.9 and 9.7 ms, 886 25.9 and 31.4, 2,000 7.7 and 9.7; 4,999
     // 11.0 and 9.2, 20,000 90.7 and 56.2.
-    lp.lanes_per_fiber = w.FA <= (uint32_t)lp.num_sms * 16u ? 32 : 8;
+    // Short fibers use one or two of eight lanes (a strip takes at least 5
+    // triplets), so they take four once 8-lane warps are more than resident:
+    // update of 64 iterations of 40,000 8-vertex fibers 15.2 against 20.5 ms
+    // with eight, 14,000 of 8 6.7 and 8.8, 20,000 of 31 22.3 and 27.8, of 60
+    // 36.1 and 39.7; but 7,000 of 8 5.9 and 5.5, 10,000 of 4 3.7 and 3.6, and
+    // longer fibers (32 iterations of 20,000 of 72) 20.4 and 20.0.
+    lp.lanes_per_fiber = w.FA <= (uint32_t)lp.num_sms * 16u ? 32
+                         : w.FA > (uint32_t)lp.num_sms * 72u && w.max_fiber > 2 && w.max_fiber <= 64 ? 4 : 8;
     if (const char *env = std::getenv("TGL_LANES_PER_FIBER")) lp.lanes_per_fiber = std::atoi(env);
     if (lp.tune_lanes) lp.lanes_per_fiber = lp.tune_lanes;
     if (lp.lanes_per_fiber != 2 && lp.lanes_per_fiber != 4 && lp.lanes_per_fiber != 8 && lp.lanes_per_fiber != 32)
@@ -2919,7 +2932,12 @@ static void enqueue_lanes(const WorldDev &w, const LaunchPlan &lp, const StepPar
     const dim3 grid(lp.lanes_blocks), block(32 * lp.lanes_wpb);
     const size_t smem = lp.lanes_smem * lp.lanes_wpb;
     switch (lp.strip_lanes) {
-        case 8: fiber_lanes_kernel<8, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
+        case 8:
+            if (w.max_fiber > 2)
+                fiber_lanes_kernel<8, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride);
+            else
+                fiber_lanes_kernel<8, A, FM, false><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride);
+            break;
         case 16: fiber_lanes_kernel<16, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
         case 32: fiber_lanes_kernel<32, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
         default: fiber_lanes_kernel<4, A, FM><<<grid, block, smem, st>>>(w, sp, lp.lanes_stride); break;
