@@ -696,19 +696,17 @@ __device__ inline void add_segment(const MpGraph &g, int32_t c, Row row, Share s
     }
 }
 
-constexpr int MP_RUN = 8;  // consecutive vertices of one warp's walk
-
-// A warp's walk over MP_RUN consecutive vertices: visit(v, links, sums) with
+// A warp's walk over `run` consecutive vertices: visit(v, links, sums) with
 // each vertex's sums over the edges into its two segments, the one before it
 // first. Consecutive vertices of a fiber share a segment, whose edges are
 // then read once for both (in the order of the sums: a vertex's second
 // segment adds to what its first gave).
 template <typename Row, typename Share, typename Visit>
-__device__ inline void walk_vertices(const MpGraph &g, int64_t first, Row row, Share share, Visit visit) {
+__device__ inline void walk_vertices(const MpGraph &g, int64_t first, int run, Row row, Share share, Visit visit) {
     const SegmentSums zero = {make_float2(0.0f, 0.0f), 0.0f};
     SegmentSums carried = zero;
     int32_t carried_segment = -1;
-    const int64_t end = first + MP_RUN < g.V ? first + MP_RUN : g.V;
+    const int64_t end = first + run < g.V ? first + run : g.V;
     for (int64_t v = first; v < end; ++v) {
         const int4 l = g.links[v];
         SegmentSums sums = zero;
@@ -729,13 +727,17 @@ __device__ inline void walk_vertices(const MpGraph &g, int64_t first, Row row, S
 
 // Per vertex: [h, the weighted mean of the messages into its two segments
 // (weights: its share, s or 1 - s), mean of the fiber neighbors' h]. Bound by
-// the messages' bytes (256 a row): 0.76 ms for 8.1 M edges (2.7 TB/s); a warp
-// per vertex, which read each message for both vertices of its segment and
-// the weights twice, took 1.02 ms. (The same walk over the edges out of a
-// vertex, whose rows lie anywhere, was slower than a warp per vertex: 0.58
-// against 0.51 ms in edge_inputs_backward_kernel.)
+// the messages' bytes (256 a row): 0.50 ms for 8.1 M edges and 200 k vertices
+// in runs of 8 (4.2 TB/s), 0.57 ms with a warp per vertex, which reads each
+// message for both vertices of its segment. Smaller graphs are bound by the
+// chain of a warp's reads, and take a vertex a warp: 100 k vertices 0.28
+// against 0.32 ms, 20 k 79 against 217 us, 6 k 27 against 85 us. (The same
+// walk over the edges out of a vertex, whose rows lie anywhere, was slower
+// than a warp per vertex: 0.58 against 0.51 ms in edge_inputs_backward_kernel.)
+constexpr int MP_RUN = 8;
+constexpr int32_t MP_RUN_VERTICES = 148 * 1024;  // fewer: a vertex a warp
 __global__ void node_inputs_kernel(MpGraph g, const float *__restrict__ h, const float *__restrict__ m,
-                                   __nv_bfloat16 *__restrict__ x) {
+                                   __nv_bfloat16 *__restrict__ x, int run) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     const auto row_of = [&](int32_t e) { return reinterpret_cast<const float2 *>(m + (int64_t)e * MP_HIDDEN)[lane]; };
@@ -767,8 +769,8 @@ __global__ void node_inputs_kernel(MpGraph g, const float *__restrict__ h, const
         row[32 + lane] = __floats2bfloat162_rn(agg.x, agg.y);
         row[64 + lane] = __floats2bfloat162_rn(nb.x, nb.y);
     };
-    for (int64_t run = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); run * MP_RUN < g.V; run += warps)
-        walk_vertices(g, run * MP_RUN, row_of, share_of, visit);
+    for (int64_t first = run * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)); first < g.V; first += run * warps)
+        walk_vertices(g, first, run, row_of, share_of, visit);
 }
 
 // dH[v] += dX[v, 0:64] + sum over fiber neighbors u of dX[u, 128:192] / count(u);
@@ -984,8 +986,10 @@ extern "C" int tgl_mp_node_inputs(const tgl_mp_graph *graph, const float *h, con
     if (tgl::bad_graph(graph) || !h || !x_node || (graph->edge_count > 0 && !m))
         return gemm_error(TGL_ERR_INVALID, "tgl_mp_node_inputs: bad arguments");
     if (graph->vertex_count == 0) return 0;
-    tgl::node_inputs_kernel<<<tgl::warps_grid(graph->vertex_count), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        tgl::view(graph), h, m, static_cast<__nv_bfloat16 *>(x_node));
+    const int run = graph->vertex_count < tgl::MP_RUN_VERTICES ? 1 : tgl::MP_RUN;
+    const int64_t runs = ((int64_t)graph->vertex_count + run - 1) / run;
+    tgl::node_inputs_kernel<<<tgl::warps_grid(runs), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        tgl::view(graph), h, m, static_cast<__nv_bfloat16 *>(x_node), run);
     return tgl::launched("tgl_mp_node_inputs");
 }
 
