@@ -1,6 +1,7 @@
 """The message kernels' results do not depend on how a graph's size splits them.
 
-A warp takes one vertex of a small graph and a run of eight of a large one.
+A warp takes one vertex of a small graph and a run of eight of a large one,
+and one to 32 edges.
 Copies of one graph side by side, in numbers around each change of the split
 and so that the copies start anywhere in a run, give each copy the bits that
 the graph gives alone.
@@ -70,7 +71,7 @@ def small(cuda_lib):
     return graph, h, m
 
 
-@pytest.mark.parametrize("vertices", [1, 20_000, 148 * 1024, 148 * 1024 + 1240, 400_000])
+@pytest.mark.parametrize("vertices", [1, 2 * 1240, 5 * 1240, 20_000, 148 * 1024, 148 * 1024 + 1240, 400_000])
 def test_copies_of_a_graph_get_its_bits(vertices, small):
     import torch
 
