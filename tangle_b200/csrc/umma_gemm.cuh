@@ -54,7 +54,7 @@ struct GemmArgs {
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_KC = 64;   // contraction elements staged per chunk
 constexpr int GEMM_THREADS = 128;
-constexpr int GEMM_STAGES = 4;  // chunks in flight
+constexpr int GEMM_STAGES = 4;  // chunks in flight, at most
 
 __device__ inline uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -81,9 +81,10 @@ __host__ __device__ inline uint32_t instr_desc_bf16(int m, int n, int a_mn, int 
 }
 
 // 16 bytes from global to shared memory, asynchronously; zeros when !valid
-// (nothing is read).
+// (nothing is read). Through L1, where the CTAs of an SM find each other's B
+// (200 k x 64 over 16: 25.7 us, 34.9 past L1).
 __device__ inline void copy_async16(uint8_t *dst, const void *src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
                  : "memory");
 }
 
@@ -91,29 +92,31 @@ __device__ inline void copy_async16(uint8_t *dst, const void *src, bool valid) {
 // into the canonical layout at `dst`; elements past k_end, and K-major rows
 // past `rows`, become zero. Every 16-byte global vector is one row of one core
 // matrix. Of an MN-major operand only the 8-row groups below `rows` are
-// copied: the others are the caller's to zero.
-__device__ inline void stage_operand(uint8_t *dst, const __nv_bfloat16 *src, int64_t ld, int mn, int R, int64_t rows,
+// copied: the others are the caller's to zero. R is ROWS, or `r` where that
+// is 0 (known row counts divide by shifts).
+template <int ROWS>
+__device__ inline void stage_operand(uint8_t *dst, const __nv_bfloat16 *src, int64_t ld, int mn, int r, int64_t rows,
                                      int64_t r0, int64_t k0, int kc, int64_t k_end) {
-    const int rgroups = R / 8;
+    const int R = ROWS ? ROWS : r, rgroups = R / 8;
+    const auto copy_group = [&](int k, int rg) {  // r = r0 + 8 rg .. +7 of contraction row k
+        const int64_t kk = k0 + k;
+        const bool valid = kk < k_end;
+        copy_async16(dst + ((k / 8) * rgroups + rg) * 128 + (k % 8) * 16, valid ? src + kk * ld + r0 + 8 * rg : src, valid);
+    };
     if (!mn) {
         // K-major: vector (r, kg) holds k = k0 + 8 kg .. +7 of row r.
         const int kgroups = kc / 8;
         for (int v = threadIdx.x; v < R * kgroups; v += blockDim.x) {
-            const int r = v / kgroups, kg = v % kgroups;
-            const int64_t row = r0 + r, kk = k0 + 8 * kg;
+            const int row_in = v / kgroups, kg = v % kgroups;
+            const int64_t row = r0 + row_in, kk = k0 + 8 * kg;
             const bool valid = row < rows && kk < k_end;
-            copy_async16(dst + (kg * rgroups + r / 8) * 128 + (r % 8) * 16, valid ? src + row * ld + kk : src, valid);
+            copy_async16(dst + (kg * rgroups + row_in / 8) * 128 + (row_in % 8) * 16, valid ? src + row * ld + kk : src, valid);
         }
+    } else if (rows - r0 >= R) {
+        for (int v = threadIdx.x; v < kc * rgroups; v += blockDim.x) copy_group(v / rgroups, v % rgroups);
     } else {
-        // MN-major: vector (k, rg) holds r = r0 + 8 rg .. +7 of contraction row k.
-        const int used = rows - r0 < R ? (int)((rows - r0 + 7) / 8) : rgroups;
-        for (int v = threadIdx.x; v < kc * used; v += blockDim.x) {
-            const int k = v / used, rg = v % used;
-            const int64_t kk = k0 + k;
-            const bool valid = kk < k_end;
-            copy_async16(dst + ((k / 8) * rgroups + rg) * 128 + (k % 8) * 16, valid ? src + kk * ld + r0 + 8 * rg : src,
-                         valid);
-        }
+        const int used = (int)((rows - r0 + 7) / 8);
+        for (int v = threadIdx.x; v < kc * used; v += blockDim.x) copy_group(v / used, v % used);
     }
 }
 
@@ -137,6 +140,9 @@ __device__ inline bool mbar_wait(uint32_t bar, uint32_t phase, unsigned int *err
 // K splits). N columns of f32 accumulator in tensor memory. GEMM_STAGES
 // contraction chunks are in flight: a chunk's buffers are refilled
 // asynchronously as soon as the MMAs of the chunk before last have read them.
+// The launch allots min(chunks, GEMM_STAGES) buffers, so that CTAs with a short
+// contraction share an SM (200 k x 128 over one chunk, both operands MN-major,
+// 57 us against 84 with four buffers and past L1).
 // The weight gradients of the nodes have a dozen splits of 8,192 rows, so each
 // CTA's chain of chunks is the time: 1.5 us a chunk (0.19 ms) against 4.9 us
 // (0.63 ms) when every chunk waited for its own loads, products and buffers;
@@ -160,13 +166,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_kernel(GemmArgs g) 
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GEMM_STAGES; ++s)
+        for (int s = 0; s < GEMM_STAGES && s < chunks; ++s)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mma_bar[s])));
         asm volatile("fence.mbarrier_init.release.cluster;");
         failed = 0;
     }
     if (g.a_mn && m0 + GEMM_BM > g.m)  // the row groups that no chunk fills
-        for (int s = 0; s < GEMM_STAGES; ++s)
+        for (int s = 0; s < GEMM_STAGES && s < chunks; ++s)
             for (uint32_t v = threadIdx.x; v < a_bytes / 16; v += blockDim.x)
                 *reinterpret_cast<uint4 *>(gemm_smem + s * stage_bytes + 16 * v) = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -185,8 +191,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_kernel(GemmArgs g) 
         if (c < chunks) {
             uint8_t *const sa = gemm_smem + (uint32_t)(c % GEMM_STAGES) * stage_bytes;
             const int64_t k0 = k_begin + c * GEMM_KC;
-            stage_operand(sa, g.a, g.lda, g.a_mn, GEMM_BM, g.m, m0, k0, length(c), k_end);
-            stage_operand(sa + a_bytes, g.b, g.ldb, g.b_mn, g.n, g.n, 0, k0, length(c), k_end);
+            stage_operand<GEMM_BM>(sa, g.a, g.lda, g.a_mn, GEMM_BM, g.m, m0, k0, length(c), k_end);
+            stage_operand<0>(sa + a_bytes, g.b, g.ldb, g.b_mn, g.n, g.n, 0, k0, length(c), k_end);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };

@@ -156,7 +156,9 @@ extern "C" int tgl_gemm_bf16(const tgl_gemm *p, void *stream) {
         const int rc = gemm_tma(p, g, static_cast<cudaStream_t>(stream));
         if (rc != 1) return rc;
     }
-    const size_t smem = (size_t)tgl::GEMM_STAGES * (tgl::GEMM_BM + p->n) * tgl::GEMM_KC * 2;
+    const int64_t longest = p->k < k_split ? p->k : k_split;  // one split's contraction
+    const int64_t chunks = std::max<int64_t>((longest + tgl::GEMM_KC - 1) / tgl::GEMM_KC, 1);
+    const size_t smem = (size_t)std::min<int64_t>(chunks, tgl::GEMM_STAGES) * (tgl::GEMM_BM + p->n) * tgl::GEMM_KC * 2;
     static std::once_flag configured;
     std::call_once(configured, [] {
         cudaFuncSetAttribute(tgl::umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
