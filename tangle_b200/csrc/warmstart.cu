@@ -61,22 +61,28 @@ bool kmajor_map(CUtensorMap *map, const void *base, int64_t rows, int64_t k, int
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Whether an MN-major B is worth keeping in each CTA's shared memory: every
+// CTA writes all of it once, which its tiles have to repay. On the staged
+// kernel and resident: 1,000 x 256 over 256 21 and 50 us, 20 k x 128 over 128
+// 15.7 and 17.8, 60 k x 192 over 16 30.6 and 33.9; but 20 k x 64 over 64 8.6 and
+// 7.2, 60 k x 128 over 64 21.3 and 17.9, 60 k x 256 over 256 80.8 and 76.8,
+// 400 k x 64 over 64 66.7 and 38.2, 400 k x 256 over 128 248 and 212.
+bool resident_pays(int64_t tiles, int n, int64_t k, int sms) {
+    if (n > 128 && k < 64) return false;
+    const int per_sm = n <= 64 ? 1 : n <= 128 || k >= n ? 3 : n <= 192 ? 4 : 16;
+    return tiles >= (int64_t)per_sm * sms;
+}
+
 // The persistent TMA kernel for products with a K-major A and an unsplit
 // contraction (an MN-major B as long as it fits in shared memory beside the
-// stages); 0 when it ran, 1 when this product or the driver calls for the
-// staged kernel instead, or an error code.
+// stages, and pays there); 0 when it ran, 1 when this product or the driver
+// calls for the staged kernel instead, or an error code.
 int gemm_tma(const tgl_gemm *p, const tgl::GemmArgs &g, cudaStream_t stream) {
     if (p->a_mn || p->k_split > 0 || p->k <= 0 || std::getenv("TGL_GEMM_STAGED")) return 1;
     if (p->m > 0x7FFFFF80 || p->k > 0x7FFFFFF0) return 1;  // TMA coordinates are 32-bit
     if (p->b_mn && p->k > 512) return 1;
     const size_t smem = p->b_mn ? tgl::tma_resident_smem_bytes(p->n, p->k) : tgl::tma_smem_bytes(p->n);
     if (smem > 220u * 1024u) return 1;
-    CUtensorMap map_a, map_b;
-    if (!kmajor_map(&map_a, p->a, p->m, p->k, p->lda, tgl::GEMM_BM)) return 1;
-    if (p->b_mn)
-        map_b = map_a;  // not read
-    else if (!kmajor_map(&map_b, p->b, p->n, p->k, p->ldb, p->n))
-        return 1;
     static std::once_flag once;
     static int sms = 0;
     std::call_once(once, [] {
@@ -87,11 +93,18 @@ int gemm_tma(const tgl_gemm *p, const tgl::GemmArgs &g, cudaStream_t stream) {
                              (int)tgl::tma_smem_bytes(256));
         cudaFuncSetAttribute(tgl::umma_gemm_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     });
+    const int64_t tiles = ((int64_t)p->m + tgl::GEMM_BM - 1) / tgl::GEMM_BM;
+    if (p->b_mn && !resident_pays(tiles, p->n, p->k, sms)) return 1;
+    CUtensorMap map_a, map_b;
+    if (!kmajor_map(&map_a, p->a, p->m, p->k, p->lda, tgl::GEMM_BM)) return 1;
+    if (p->b_mn)
+        map_b = map_a;  // not read
+    else if (!kmajor_map(&map_b, p->b, p->n, p->k, p->ldb, p->n))
+        return 1;
     int cols = 32;
     while (cols < p->n) cols <<= 1;
     const int by_smem = (int)((220u * 1024u) / smem), by_tmem = 512 / (2 * cols);
     const int per_sm = std::max(1, std::min(by_smem, by_tmem));
-    const int64_t tiles = ((int64_t)p->m + tgl::GEMM_BM - 1) / tgl::GEMM_BM;
     const int blocks = (int)std::min<int64_t>(tiles, (int64_t)std::max(sms, 1) * per_sm);
     if (p->b_mn)
         tgl::umma_gemm_tma_kernel<true><<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
