@@ -22,11 +22,10 @@
 #include "kernels.cuh"
 #include "formation.cuh"
 #include "contact.cuh"
+#include "dynamic_smem.h"
 
 #include <algorithm>
 #include <cstdlib>
-#include <map>
-#include <mutex>
 
 namespace tgl {
 
@@ -2673,20 +2672,9 @@ int grid_for(uint64_t n, int threads, int cap) {
 
 }  // namespace
 
-// A kernel's largest dynamic shared memory is a process-wide attribute of
-// the function, shared by every world: raise it when a plan needs more, and
-// never lower it below what another world (or an earlier plan of this one,
-// whose captured graphs may still launch) needs.
 template <typename Kernel>
 static void allow_dynamic_smem(Kernel kernel, size_t bytes) {
-    static std::mutex lock;
-    static std::map<const void *, size_t> granted;
-    const void *key = reinterpret_cast<const void *>(kernel);
-    std::lock_guard<std::mutex> guard(lock);
-    size_t &current = granted[key];
-    if (bytes <= current) return;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
-        current = bytes;
+    allow_dynamic_smem(reinterpret_cast<const void *>(kernel), bytes);
 }
 
 void plan_contact_pass(const WorldDev &w, LaunchPlan &lp, int per_sm) {

@@ -11,6 +11,7 @@
 #include <mutex>
 
 #include "../../include/tangle_cuda.h"
+#include "dynamic_smem.h"
 #include "umma_gemm.cuh"
 #include "umma_gemm_tma.cuh"
 
@@ -83,16 +84,9 @@ int gemm_tma(const tgl_gemm *p, const tgl::GemmArgs &g, cudaStream_t stream) {
     if (p->b_mn && p->k > 512) return 1;
     const size_t smem = p->b_mn ? tgl::tma_resident_smem_bytes(p->n, p->k) : tgl::tma_smem_bytes(p->n);
     if (smem > 220u * 1024u) return 1;
-    static std::once_flag once;
-    static int sms = 0;
-    std::call_once(once, [] {
-        int device = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaFuncSetAttribute(tgl::umma_gemm_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)tgl::tma_smem_bytes(256));
-        cudaFuncSetAttribute(tgl::umma_gemm_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    });
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int64_t tiles = ((int64_t)p->m + tgl::GEMM_BM - 1) / tgl::GEMM_BM;
     if (p->b_mn && !resident_pays(tiles, p->n, p->k, sms)) return 1;
     CUtensorMap map_a, map_b;
@@ -106,10 +100,10 @@ int gemm_tma(const tgl_gemm *p, const tgl::GemmArgs &g, cudaStream_t stream) {
     const int by_smem = (int)((220u * 1024u) / smem), by_tmem = 512 / (2 * cols);
     const int per_sm = std::max(1, std::min(by_smem, by_tmem));
     const int blocks = (int)std::min<int64_t>(tiles, (int64_t)std::max(sms, 1) * per_sm);
-    if (p->b_mn)
-        tgl::umma_gemm_tma_kernel<true><<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
-    else
-        tgl::umma_gemm_tma_kernel<false><<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
+    const auto kernel = p->b_mn ? tgl::umma_gemm_tma_kernel<true> : tgl::umma_gemm_tma_kernel<false>;
+    static tgl::DynamicSmem allowed[2];
+    allowed[p->b_mn ? 1 : 0].allow(reinterpret_cast<const void *>(kernel), smem);
+    kernel<<<blocks, tgl::TMA_GEMM_THREADS, smem, stream>>>(map_a, map_b, g);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return gemm_error(TGL_ERR_CUDA, std::string("tgl_gemm_bf16: ") + cudaGetErrorString(e));
     return 0;
@@ -172,11 +166,8 @@ extern "C" int tgl_gemm_bf16(const tgl_gemm *p, void *stream) {
     const int64_t longest = p->k < k_split ? p->k : k_split;  // one split's contraction
     const int64_t chunks = std::max<int64_t>((longest + tgl::GEMM_KC - 1) / tgl::GEMM_KC, 1);
     const size_t smem = (size_t)std::min<int64_t>(chunks, tgl::GEMM_STAGES) * (tgl::GEMM_BM + p->n) * tgl::GEMM_KC * 2;
-    static std::once_flag configured;
-    std::call_once(configured, [] {
-        cudaFuncSetAttribute(tgl::umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             tgl::GEMM_STAGES * (tgl::GEMM_BM + 256) * tgl::GEMM_KC * 2);
-    });
+    static tgl::DynamicSmem allowed;
+    allowed.allow(reinterpret_cast<const void *>(tgl::umma_gemm_kernel), smem);
     dim3 grid((unsigned)((p->m + tgl::GEMM_BM - 1) / tgl::GEMM_BM), (unsigned)splits);
     tgl::umma_gemm_kernel<<<grid, tgl::GEMM_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(g);
     cudaError_t e = cudaGetLastError();
