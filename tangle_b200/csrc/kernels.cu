@@ -2724,14 +2724,19 @@ void plan_launches(const WorldDev &w, LaunchPlan &lp) {
     // round's instructions). Update of a batch with 32 lanes and with 8: 40
     // fibers 7.9 and 9.7 ms, 886 25.9 and 31.4, 2,000 7.7 and 9.7; 4,999
     // 11.0 and 9.2, 20,000 90.7 and 56.2.
-    // Short fibers use one or two of eight lanes (a strip takes at least 5
+    // Short fibers use one to three of eight lanes (a strip takes at least 5
     // triplets), so they take four once 8-lane warps are more than resident:
-    // update of 64 iterations of 40,000 8-vertex fibers 15.2 against 20.5 ms
-    // with eight, 14,000 of 8 6.7 and 8.8, 20,000 of 31 22.3 and 27.8, of 60
-    // 36.1 and 39.7; but 7,000 of 8 5.9 and 5.5, 10,000 of 4 3.7 and 3.6, and
-    // longer fibers (32 iterations of 20,000 of 72) 20.4 and 20.0.
+    // update of 64 iterations with four and with eight lanes of 40,000 bent
+    // 8-vertex fibers 15.2 and 20.5 ms, 14,000 of 8 6.7 and 8.8, 30,000 of 31
+    // 28.8 and 38.7; straight ones, which only scan, 6.9 and 6.7, 7.5 and 7.5.
+    // But 7,000 of 8 5.9 and 5.5, 10,000 of 4 3.7 and 3.6, and 20,000 straight
+    // ones of 48 10.6 and 8.7 (bent 31.1 and 36.2: there the lanes' longer
+    // strips start to cost what their sharing saves). An arena's kernel has
+    // half again as many warps resident: 40 specimens of 1,000 bent fibers of
+    // 16 10.3 and 14.0, of 24 13.1 and 17.1, of straight ones of 31 5.0 and 4.4.
+    const uint32_t short_fiber = lp.arena ? 24 : 32;
     lp.lanes_per_fiber = w.FA <= (uint32_t)lp.num_sms * 16u ? 32
-                         : w.FA > (uint32_t)lp.num_sms * 72u && w.max_fiber > 2 && w.max_fiber <= 64 ? 4 : 8;
+                         : w.FA > (uint32_t)lp.num_sms * 72u && w.max_fiber > 2 && w.max_fiber <= short_fiber ? 4 : 8;
     if (const char *env = std::getenv("TGL_LANES_PER_FIBER")) lp.lanes_per_fiber = std::atoi(env);
     if (lp.tune_lanes) lp.lanes_per_fiber = lp.tune_lanes;
     if (lp.lanes_per_fiber != 2 && lp.lanes_per_fiber != 4 && lp.lanes_per_fiber != 8 && lp.lanes_per_fiber != 32)

@@ -1,7 +1,7 @@
 """Worlds of many short fibers: the update's default lanes, and its results.
 
-From 72 fibers per SM, fibers of 3 to 64 vertices take four lanes each by
-default (eight before); worlds of two-vertex fibers, which have nothing to
+From 72 fibers per SM, fibers of 3 to 32 vertices (24 in an arena) take four
+lanes each by default (eight before); worlds of two-vertex fibers, which have nothing to
 sweep, run a kernel without the sweeps. Positions and curvature maxima are
 the oracle's bit for bit, in a periodic box and between walls, and an
 arena's are those of its specimens alone.
@@ -39,7 +39,7 @@ def settings():
 
 
 @pytest.mark.parametrize("per_sm, vertices, lanes", [(16, 8, 32), (17, 8, 8), (72, 8, 8), (73, 8, 4), (73, 3, 4), (73, 2, 8),
-                                                     (73, 64, 4), (73, 65, 8)])
+                                                     (73, 32, 4), (73, 33, 8)])
 def test_default_lanes(per_sm, vertices, lanes, cuda_lib):
     import torch
 
@@ -66,6 +66,18 @@ def test_short_fibers_match_the_oracle(count, vertices, periodic, cuda_lib):
         np.testing.assert_array_equal(dev.wall_reactions().view(np.uint32), orc.wall_reactions().view(np.uint32))
     dev.close()
     orc.close()
+
+
+@pytest.mark.parametrize("vertices, lanes", [(24, 4), (25, 8)])
+def test_default_lanes_of_an_arena(vertices, lanes, cuda_lib):
+    import torch
+
+    from tangle_b200.device import DeviceWorld
+
+    count = 73 * torch.cuda.get_device_properties(0).multi_processor_count // 4
+    arena = DeviceWorld.arena([short_fibers(count + 1, vertices, seed=s) for s in range(4)], CELLS, 5.0e-7)
+    assert arena.launch_params()["lanes_per_fiber"] == lanes
+    arena.close()
 
 
 def test_two_vertex_specimens_of_an_arena(cuda_lib):
