@@ -285,9 +285,10 @@ def issue_bound(profile: str, refresh_share=None):
     launch over the same launch's duration, against 4 warp instructions per
     clock on each of the 148 SMs at the 1,965 MHz the capture ran at; for the
     contact pass, listed and refresh passes weighted by their share of this
-    run's passes. Both figures come from the same launches (the capture's
-    state, early in the trajectory), so the fraction does not mix states
-    with this run's timing. None without the capture."""
+    run's passes. Both figures come from the same launches (after 1,280
+    iterations from the initial specimen, narrow contact lists), so the
+    fraction does not mix states with this run's timing. None without the
+    capture."""
     path = os.path.join(ROOT, "profiles", profile)
     try:
         with open(path) as fh:

@@ -185,17 +185,19 @@ int tgl_neighbor_list_rebuilds(tgl_world *world, uint32_t *rebuilds);
 
 /* Contact lists (no reference counterpart: an internal second level under
  * the Verlet lists that changes no result). Each cell-list slot keeps the
- * entries of its segment's Verlet list that lie within `contact_skin` of
- * touching at a snapshot of the positions, in the Verlet list's order; the
- * contact pass reads them instead of the Verlet list until some vertex moves
- * more than contact_skin / 2 from the snapshot or the Verlet lists are
- * rebuilt. The skin is 0.1 of the neighbor skin unless the environment
- * variable TGL_CONTACT_SKIN, read when a world is created, gives another
- * fraction in (0, 1] (0 turns them off); they are also off when a periodic
- * box edge is under about four segment lengths plus four radii, and every
- * pass reads the Verlet lists while some segment is stretched that far.
- * Reports the skin (0 when off), the entries per slot, and the refreshes
- * done so far. */
+ * entries of its segment's Verlet list that lie within a skin of touching at
+ * a snapshot of the positions, in the Verlet list's order; the contact pass
+ * reads them instead of the Verlet list until some vertex moves more than
+ * half that skin from the snapshot or the Verlet lists are rebuilt. Each
+ * refresh makes its lists (in an arena, each specimen's) with `contact_skin`
+ * or, while the positions move fast and the box leaves room, 2.5 times that
+ * (at most the neighbor skin). contact_skin is 0.1 of the neighbor skin
+ * unless the environment variable TGL_CONTACT_SKIN, read when a world is
+ * created, gives another fraction in (0, 1] (0 turns the lists off); they are
+ * also off when a periodic box edge is under about four segment lengths plus
+ * four radii, and every pass reads the Verlet lists while some segment is
+ * stretched that far. Reports contact_skin (the narrow one; 0 when off), the
+ * entries per slot, and the refreshes done so far. */
 int tgl_contact_list_info(tgl_world *world, float *contact_skin, uint32_t *block, uint32_t *refreshes);
 
 /* DeviceFiberWorld::capture_contacts (world.rs:2195-2335) with
@@ -365,8 +367,10 @@ typedef struct {
  * for bit, and the same gate decisions; they only move time between
  * kernels. */
 typedef struct {
-    uint32_t lanes_per_fiber;       /* lanes per fiber in the curvature sweeps: 2, 4, 8 or 32 */
-    uint32_t contact_blocks_per_sm; /* contact-pass blocks per SM (256 threads each): 1, 2 or 3 */
+    uint32_t lanes_per_fiber;       /* lanes per fiber in the curvature sweeps: 2, 4, 8 or 32 (as asked for:
+                                        2 runs as 4, and any is raised until the longest fiber fits) */
+    uint32_t contact_blocks_per_sm; /* contact-pass blocks per SM (256 threads each), at most: 1, 2 or 3
+                                        (untuned, the least with the plan in use is reported) */
     uint32_t build_chunk;           /* candidate slots a Verlet-build block stages at once: 512 to 4096 */
     float contact_skin_fraction;    /* contact-list skin over the neighbor skin: 0 (lists off) or (0, 1];
                                        above 0 only where the world allocated contact lists */
@@ -387,9 +391,10 @@ typedef struct {
     float best_ms;              /* the chosen parameters, per trial batch */
 } tgl_autotune_report;
 
-/* Searches the launch parameters one at a time (coordinate descent over the
- * candidate sets above, starting from the world's current ones), timing
- * each candidate with CUDA events on a batch of `trial_iterations`
+/* Searches the launch parameters one at a time (coordinate descent over
+ * candidates of each, starting from the world's current plan; candidates that
+ * give a plan already timed are skipped), timing each candidate with CUDA
+ * events on a batch of `trial_iterations`
  * iterations of `config` (force_full_iterations implied), best of two after
  * one untimed batch that captures its graph. Every trial starts from the
  * world's state at the call: positions, last steps, formation commands and

@@ -1899,8 +1899,10 @@ __device__ inline bool project_triplet(float4 &q0, float4 &q1, float4 &q2, bool 
 // positions).
 //
 // What bounds it: the projection's chain (about 290 instructions, 730 cycles
-// on a lone warp) times the longest run of triplets that wait for each other,
-// and instruction issue where the chip is full. The former sweep applied one
+// on a lone warp) times the longest run of triplets that wait for each other;
+// where the chip is full, those chains at 16 warps an SM, which the registers
+// and the staged records both leave (the update of 20,000 fibers of 108 takes
+// 0.45 to 0.51 of the issue slots). The former sweep applied one
 // acting triplet of 8 tested ones per round and fiber: 25-42 rounds per
 // update on 31-vertex fibers, 130-150 on the mid-size specimen's and 465 on
 // 180-vertex ply fibers; strips take 6-20, 28-39 and 145-185. Update stage

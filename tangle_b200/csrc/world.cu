@@ -819,8 +819,7 @@ int build_world(std::vector<HostSpecimen> &hosts, const tgl_cell_list_config *cl
     d.grid = grid;
     // Contact lists: on by default at a tenth of the skin (TGL_CONTACT_SKIN
     // sets the fraction, 0 turns them off); in an arena one contact skin
-    // serves every specimen (a tenth of the smallest neighbor skin) and one
-    // refresh flag covers them all.
+    // serves every specimen (a tenth of the smallest neighbor skin).
     float contact_fraction = 0.1f;
     if (const char *env = std::getenv("TGL_CONTACT_SKIN")) contact_fraction = std::strtof(env, nullptr);
     if (!(contact_fraction > 0.0f && contact_fraction <= 1.0f) || !(w->contact_skin_base > 0.0f))
