@@ -758,7 +758,8 @@ def run_cuda(args):
                         "algorithmic_bytes_per_launch": algorithmic, "avg_launch_ms": avg_contact_s * 1000.0,
                         "contact_passes": contact_passes, "refresh_passes": refreshes,
                         "contact_skin_m": contact_info["skin"]}
-    if not batched and contact_info["block"] > 0:
+    captured = args.workload == "mid_size" and args.scale == 1.0  # the committed capture's workload
+    if captured and contact_info["block"] > 0:
         roofline_contact["issue_bound"] = issue_bound("contact_traffic.json", refresh_share)
     # Roofline of the fiber update, the largest kernel (about 55 % of the
     # step): its algorithmic bytes per launch over its mean duration.
@@ -772,7 +773,7 @@ def run_cuda(args):
                 "kernel": "fiber_lanes_kernel (internal, contact and curvature corrections)",
                 "algorithmic_bytes_per_launch": update_algorithmic, "avg_launch_ms": avg_update_s * 1000.0,
                 "launches": updates}
-    if not batched:
+    if captured:
         roofline["issue_bound"] = issue_bound("update_traffic.json")
 
     # End to end through the public API with pinned host buffers: the timed
