@@ -2681,13 +2681,14 @@ static void allow_dynamic_smem(Kernel kernel, size_t bytes) {
 
 void plan_contact_pass(const WorldDev &w, LaunchPlan &lp, int per_sm) {
     const uint32_t batches = (w.NS + 31) / 32, resident = (uint32_t)(lp.num_sms * per_sm) * CONTACT_WARPS;
-    // Four warps share a batch's segments while each batch could have a warp
-    // of its own (a warp's chain of rounds is then the pass): contact stage of
-    // 40 31-vertex fibers 2.44 -> 2.22 ms per 128 iterations, of 357-vertex
-    // ones 2.61 -> 2.37, of 886 of 66 and 180 4.51 -> 4.33. With 1.7 batches a
-    // warp or more, the fuller rounds of whole batches win: 6.21 ms against
-    // 7.69 with four and 6.58 with two (2,000 of 108, relaxed).
-    lp.contact_split = !lp.arena && batches <= resident ? 2 : 0;
+    // Four warps share a batch's segments while the batches are at most half
+    // the resident warps (a warp's chain of rounds is then the pass): contact
+    // stage with one and with four of 37 batches 2.34 and 1.87 ms per 128
+    // iterations, of 843 1.60 and 1.36 per 64, of 1,640 (long fibers) 2.59 and
+    // 2.37 per 32, of 1,312 1.51 and 1.49, sparse 1.02 and 1.13. With more,
+    // the fuller rounds of whole batches win: 2,288 4.35 and 4.38, 3,187 1.63
+    // and 1.99, 2,754 sparse ones 0.75 and 0.95.
+    lp.contact_split = !lp.arena && 2u * batches <= resident ? 2 : 0;
     lp.contact_blocks = grid_for((uint64_t)batches << lp.contact_split, CONTACT_WARPS, lp.num_sms * per_sm);
 }
 

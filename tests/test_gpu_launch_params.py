@@ -2,8 +2,8 @@
 
 Setting what launch_params() reports must leave the contact pass's grid and
 the sharing of its batches as they are. A world of b batches of 32 segments
-shares each among four warps while b is at most the resident warps (8 per
-block, p blocks per SM), in min(ceil(4 b / 8 or b / 8), p x SMs) blocks;
+shares each among four warps while b is at most half the resident warps (8
+per block, p blocks per SM), in min(ceil(4 b / 8 or b / 8), p x SMs) blocks;
 untuned, p is 3. The least p with the same plan is reported, and again once
 it has been set.
 """
@@ -37,7 +37,7 @@ def test_set_of_get_leaves_the_contact_plan(batches, cuda_lib):
     b = (world.segment_count + 31) // 32
 
     def plan(p):
-        shared = 4 if b <= 8 * p * sms else 1
+        shared = 4 if 2 * b <= 8 * p * sms else 1
         return min(-(-b * shared // 8), p * sms), shared
 
     params = world.launch_params()
