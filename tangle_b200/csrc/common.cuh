@@ -80,20 +80,28 @@ __device__ inline float reciprocal_plain(float b) {
 }
 
 // RN(a / b) from y = RN(1 / b), for |a|, b in [PLAIN_MIN, PLAIN_MAX] and a
-// quotient in [2^-120, 2^120] (a = +0 too): the division by a correctly rounded reciprocal of
-// P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34 (1990). The first correction
-// makes q faithful, so the second residual a - b q is exact and the last FMA
-// rounds a / b + d with |d| <= b 2^-49 (b scaled to [1, 2)), below the
-// distance 2^-47 / b that a quotient of 24-bit numbers keeps from every
+// quotient in [2^-120, 2^120], or a zero of either sign (the residual b q - a
+// of a zero is +0, which leaves q's sign): the division by a correctly
+// rounded reciprocal of P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990). The first
+// correction makes q faithful, so the second residual b q - a is exact and the
+// last FMA rounds a / b + d with |d| <= b 2^-49 (b scaled to [1, 2)), below
+// the distance 2^-47 / b that a quotient of 24-bit numbers keeps from every
 // rounding boundary.
 __device__ inline float div_plain(float a, float b, float y) {
     float q = __fmul_rn(a, y);
-    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    q = __fmaf_rn(-__fmaf_rn(b, q, -a), y, q);
+    return __fmaf_rn(-__fmaf_rn(b, q, -a), y, q);
 }
 
 __device__ inline float min3_abs(float x, float y, float z) { return fminf(fminf(fabsf(x), fabsf(y)), fabsf(z)); }
+
+// Whether x, y and z are each zero or at least PLAIN_MIN in magnitude: twice
+// the bits without the sign, less one, take zeros to the top.
+__device__ inline bool zero_or_plain(float x, float y, float z) {
+    const auto rank = [](float v) { return 2u * __float_as_uint(v) - 1u; };
+    return min(min(rank(x), rank(y)), rank(z)) >= 2u * __float_as_uint(PLAIN_MIN) - 1u;
+}
 #endif
 
 // f32 arc cosine with one fixed rounding sequence, so that every build of
