@@ -883,6 +883,10 @@ __device__ inline void lists_made(const WorldDev &w, Control *c) {
 // Verlet lists plus a refresh of the contact lists and their snapshot
 // (CONTACT_REFRESH, run when the refresh flag is set); the contact lists
 // (CONTACT_LISTED, run when it is clear).
+// Verlet lists with fewer entries than this may overflow at usual densities
+// (about forty neighbors); segments whose list did scan their cells.
+constexpr uint32_t SHORT_BLOCK = 64;
+
 enum { CONTACT_FULL = 0, CONTACT_REFRESH = 1, CONTACT_LISTED = 2 };
 
 // find_segment_corrections (contact.rs:232-902) over warp-owned batches of 32
@@ -978,8 +982,10 @@ __global__ void __launch_bounds__(256, 3) contact_kernel(WorldDev w, StepParams 
     // stride too: their records stay in L2 in any order, and four times the
     // takes queued on the counter: 128 passes of 20,000 two-vertex fibers 2.04
     // ms before batches were shared, 2.24 with the counter, 1.98 without; of
-    // 300 sparse ones of 108 2.19, 2.33 and 2.02.
-    const bool fixed = A || shift > 0u || parts <= stride;
+    // 300 sparse ones of 108 2.19, 2.33 and 2.02. Parts that scan cells differ
+    // too much in length for that (3,356 batches with 8 entries 71.5 ms before
+    // sharing, 46.1 with the counter, 55.6 without).
+    const bool fixed = A || parts <= stride || (shift > 0u && block >= SHORT_BLOCK);
     for (uint32_t part = fixed ? blockIdx.x * CONTACT_WARPS + warp : take_part(); part < parts;
          part = fixed ? part + stride : take_part()) {
         const uint32_t base = (part >> shift) * 32u;
@@ -2707,13 +2713,17 @@ static void allow_dynamic_smem(Kernel kernel, size_t bytes) {
 void plan_contact_pass(const WorldDev &w, LaunchPlan &lp, int per_sm) {
     const uint32_t batches = (w.NS + 31) / 32, resident = (uint32_t)(lp.num_sms * per_sm) * CONTACT_WARPS;
     // Four warps share a batch's segments while the batches are at most half
-    // the resident warps (a warp's chain of rounds is then the pass): contact
+    // the resident warps, or all of them with short lists (a warp's chain of rounds is then the pass): contact
     // stage with one and with four of 37 batches 2.34 and 1.87 ms per 128
     // iterations, of 843 1.60 and 1.36 per 64, of 1,640 (long fibers) 2.59 and
     // 2.37 per 32, of 1,312 1.51 and 1.49, sparse 1.02 and 1.13. With more,
     // the fuller rounds of whole batches win: 2,288 4.35 and 4.38, 3,187 1.63
-    // and 1.99, 2,754 sparse ones 0.75 and 0.95.
-    lp.contact_split = !lp.arena && 2u * batches <= resident ? 2 : 0;
+    // and 1.99, 2,754 sparse ones 0.75 and 0.95. Where the lists are short of
+    // the usual forty entries, segments may scan their cells, a warp each: with
+    // 8 entries 3,187 batches 23.8 and 18.7 ms per 32, 2,000 22.5 and 16.1 (with
+    // 24 entries, that most lists fit, 0.98 and 1.06).
+    const uint32_t shared = w.block < SHORT_BLOCK ? batches : 2u * batches;
+    lp.contact_split = !lp.arena && shared <= resident ? 2 : 0;
     lp.contact_blocks = grid_for((uint64_t)batches << lp.contact_split, CONTACT_WARPS, lp.num_sms * per_sm);
 }
 

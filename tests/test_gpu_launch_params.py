@@ -3,9 +3,9 @@
 Setting what launch_params() reports must leave the contact pass's grid and
 the sharing of its batches as they are. A world of b batches of 32 segments
 shares each among four warps while b is at most half the resident warps (8
-per block, p blocks per SM), in min(ceil(4 b / 8 or b / 8), p x SMs) blocks;
-untuned, p is 3. The least p with the same plan is reported, and again once
-it has been set.
+per block, p blocks per SM; all of them with lists of fewer than 64 entries),
+in min(ceil(4 b / 8 or b / 8), p x SMs) blocks; untuned, p is 3. The least p
+with the same plan is reported, and again once it has been set.
 """
 
 import numpy as np
@@ -27,17 +27,18 @@ def straight_pairs(segments):
 
 
 @pytest.mark.parametrize("batches", [5, 295, 300, 590, 940, 1180, 1190, 2400, 3600, 4800])
-def test_set_of_get_leaves_the_contact_plan(batches, cuda_lib):
+@pytest.mark.parametrize("capacity", [16, 64])
+def test_set_of_get_leaves_the_contact_plan(batches, capacity, cuda_lib):
     import torch
 
     from tangle_b200.device import DeviceWorld
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    world = DeviceWorld(straight_pairs(batches * 32), CellListConfig(neighbor_capacity=16, max_list_bytes=1 << 28), 1.0e-6)
+    world = DeviceWorld(straight_pairs(batches * 32), CellListConfig(neighbor_capacity=capacity, max_list_bytes=1 << 28), 1.0e-6)
     b = (world.segment_count + 31) // 32
 
     def plan(p):
-        shared = 4 if 2 * b <= 8 * p * sms else 1
+        shared = 4 if (1 if capacity < 64 else 2) * b <= 8 * p * sms else 1
         return min(-(-b * shared // 8), p * sms), shared
 
     params = world.launch_params()
